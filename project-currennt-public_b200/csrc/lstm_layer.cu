@@ -233,7 +233,9 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
     //   dW_rec[g][d](k, j) = sum_f h_d[k; f -/+ P] * delta_g,d[j; f], skipping the first (last) timestep
     {
         Phase ph(*this, "lstm_dw_rec_gemm");
-        const bool tc_rec = tc && (els % 4) == 0 && gemm_wants_tc(1, ls, 4 * ls, 1, els, els, K);
+        // the boxes of both operands start at column g*ls + d*els: a TMA copy must start on a 16-byte boundary (8 halves,
+        // 4 floats), other unit counts take the FFMA kernel
+        const bool tc_rec = tc && (els % (tcrec_used ? 4 : 8)) == 0 && gemm_wants_tc(1, ls, 4 * ls, 1, els, els, K);
         bool done = false;
         if (tc_rec && 4 * D <= 8) {
             // all 4*D products in ONE batched launch: batch = (direction, gate); K is split so that the

@@ -516,3 +516,17 @@ def test_a_wait_that_nothing_satisfies_runs_out_and_leaves_the_context_usable():
     want = run_kind(checker(), layers, 4, lens, x, tg, w)
     got = run_gpu(layers, 4, lens, x, tg, w, VARIANTS[2])
     parity.compare_run(layers, got, want, "after the timed-out wait", lstm_pad_zero_lens=lens)
+
+
+@pytest.mark.parametrize("ls,bi,P,lens", [(200, 1, 8, [60] * 6 + [33, 21]), (100, 0, 12, [50] * 12), (180, 1, 5, [70, 64, 31, 70, 2])])
+def test_unit_counts_of_4_modulo_8(ls, bi, P, lens):
+    """Units per direction whose gate blocks start off the 16-byte boundary of the fp16 operand copies (100, 90): the
+    recurrent weight gradient must not start its TMA boxes there."""
+    from b2lstm import workloads
+    layers = L(("input", 24), ("blstm" if bi else "lstm", ls), ("feedforward_identity", 8), ("sse", 8))
+    lens = np.array(lens, np.int32)
+    x, tg = workloads.make_fraction(24, 8, P, lens, 81, 82)
+    w = workloads.make_weights(layers, 83, 0.05)
+    want = run_kind(checker(), layers, P, lens, x, tg, w)
+    got = run_gpu(layers, P, lens, x, tg, w, VARIANTS[2])
+    parity.compare_run(layers, got, want, "ls%d bi%d P%d" % (ls, bi, P), lstm_pad_zero_lens=lens)
