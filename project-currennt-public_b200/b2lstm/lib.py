@@ -367,7 +367,8 @@ class Net:
     def set_force_ffma(self, on):
         _check(lib().b2_net_set_force_ffma(self.h, int(on)))
 
-    RECURRENCE_PATHS = {0: "stepwise", 1: "persistent_ffma", 3: "tensor_core_per_step", 5: "persistent_tensor_core"}
+    RECURRENCE_PATHS = {0: "stepwise", 1: "persistent_ffma", 3: "tensor_core_per_step", 5: "persistent_tensor_core",
+                        7: "cluster_tensor_core"}
 
     def recurrence_path(self, layer, backward=False):
         """which recurrence kernels layer `layer` really ran in its last sweep (-1: not a (b)lstm layer / none yet)"""

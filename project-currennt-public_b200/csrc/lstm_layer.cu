@@ -132,9 +132,14 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
     }
     {
         Phase ph(*this, "lstm_fwd_recurrence");
-        B2_TRY(lstm_prepare_wrecT(s, w, bufs.wrecT, st));
         int rc = 1;
-        ptc_used = want_ptc();
+        cluster_used = want_cluster();
+        if (cluster_used) {
+            rc = lstm_cluster_sweep(false, s, bufs, w, y, nullptr, status_dev, st);
+            fwd_path = 7;
+            if (rc == 1) cluster_used = false;
+        }
+        ptc_used = !cluster_used && want_ptc();
         if (ptc_used) {
             B2_TRY(ensure_ptc());
             B2_TRY(lstm_ptc_prepare(s, w, ptc, st));
@@ -142,8 +147,10 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
             fwd_path = 5;
             if (rc == 1) ptc_used = false;
         }
-        tcrec_used = !ptc_used && want_tc_recurrence();
-        if (ptc_used) {
+        tcrec_used = !cluster_used && !ptc_used && want_tc_recurrence();
+        const bool plain = !cluster_used && !ptc_used && !tcrec_used;
+        if (plain) B2_TRY(lstm_prepare_wrecT(s, w, bufs.wrecT, st));
+        if (cluster_used || ptc_used) {
         } else if (tcrec_used) {
             B2_TRY(ensure_tcrec());
             rc = lstm_forward_tc(s, bufs, tcrec, w, y, status_dev, st);
@@ -169,7 +176,10 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
     {
         Phase ph(*this, "lstm_bwd_recurrence");
         int rc = 1;
-        if (ptc_used && recurrence_mode != 6) {
+        if (cluster_used) {
+            rc = lstm_cluster_sweep(true, s, bufs, w, nullptr, dy, status_dev, st);
+            bwd_path = 7;
+        } else if (ptc_used && recurrence_mode != 6) {
             rc = lstm_ptc_sweep(true, s, bufs, ptc, w, nullptr, dy, status_dev, &tag_next, st);
             bwd_path = 5;
         }
@@ -312,6 +322,16 @@ bool LstmLayerImpl::want_tc_recurrence() const {
     const int items = s.D * ((s.P + ps - 1) / ps);
     const int passes = (items + slots - 1) / slots;
     return passes * (1.4 + 0.27 * ps) > 12.0;
+}
+
+// The register-resident cluster kernels serve up to 320 units per direction.  For one or two sequences of the unit counts that
+// have an FFMA geometry those kernels have the shorter step: an MMA always runs 8 sequences.
+bool LstmLayerImpl::want_cluster() const {
+    if (force_ffma || recurrence_mode != 1) return false;
+    const LstmShape s = shape();
+    int JB;
+    if (s.P < 3 && persistent_geometry(s.els, &JB)) return false;
+    return lstm_cluster_supported(s);
 }
 
 // The persistent tensor-core kernels serve 512 units per direction.  Modes 5 and 6 force them; the default (mode 1)

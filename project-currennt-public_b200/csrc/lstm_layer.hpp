@@ -33,10 +33,12 @@ struct LstmLayerImpl {
     // persistent tensor-core recurrence: weight images, exchange words (allocated on first use)
     PtcBuffers ptc{};
     bool ptc_used = false;        // this fraction's forward sweep ran on the persistent tensor-core kernels
+    bool cluster_used = false;    // this fraction's forward sweep ran on the register-resident cluster kernels
+    bool want_cluster() const;
     bool want_ptc() const;
     int ensure_ptc();
     // which recurrence the last forward / backward sweep actually ran: 0 one launch per timestep, 1 persistent
-    // FFMA kernels, 3 tensor-core GEMM + gate kernel per timestep, 5 persistent tensor-core kernels
+    // FFMA kernels, 3 tensor-core GEMM + gate kernel per timestep, 5 persistent tensor-core kernels, 7 register-resident cluster kernels
     int fwd_path = -1, bwd_path = -1;
     bool want_tc_recurrence() const;
     int ensure_tcrec();

@@ -530,3 +530,27 @@ def test_unit_counts_of_4_modulo_8(ls, bi, P, lens):
     want = run_kind(checker(), layers, P, lens, x, tg, w)
     got = run_gpu(layers, P, lens, x, tg, w, VARIANTS[2])
     parity.compare_run(layers, got, want, "ls%d bi%d P%d" % (ls, bi, P), lstm_pad_zero_lens=lens)
+
+
+@pytest.mark.parametrize("els,bi,P,T", [(1, 1, 3, 3), (15, 0, 4, 6), (33, 1, 8, 9), (64, 1, 9, 7), (65, 0, 17, 6), (96, 1, 33, 5), (128, 0, 4, 12),
+                                        (129, 1, 5, 9), (160, 1, 8, 11), (192, 0, 70, 6), (224, 1, 12, 7), (255, 1, 20, 6), (256, 1, 32, 9),
+                                        (256, 0, 3, 1), (256, 1, 260, 3), (257, 1, 9, 7), (320, 1, 40, 5), (300, 0, 6, 2), (48, 1, 600, 4)])
+def test_cluster_recurrence(els, bi, P, T):
+    """The register-resident cluster kernels: unit counts around the paddings of every cluster geometry, sequence counts that do not
+    fill a tile of 8, more work items than clusters fit, ragged lengths (a tile whose sequences all end early included)."""
+    from b2lstm import workloads
+    ls = els * (2 if bi else 1)
+    layers = L(("input", 7), ("blstm" if bi else "lstm", ls), ("feedforward_identity", 5), ("sse", 5))
+    lens = np.array(sorted([max(1, T - (p * 7) % (T + 1)) for p in range(P)], reverse=True), np.int32)
+    lens[0] = T
+    x, tg = workloads.make_fraction(7, 5, P, lens, 91, 92)
+    w = workloads.make_weights(layers, 93, 0.2 if els < 100 else 0.08)
+    want = run_kind(checker(), layers, P, lens, x, tg, w)
+    paths = {}
+    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0), paths=paths)
+    assert paths[1] == ("cluster_tensor_core", "cluster_tensor_core"), paths
+    parity.compare_run(layers, got, want, "els%d bi%d P%d" % (els, bi, P), lstm_pad_zero_lens=lens)
+    again = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0))
+    for key in got:
+        if key != "launches":
+            assert np.array_equal(np.asarray(got[key]), np.asarray(again[key])), "not deterministic: " + key
