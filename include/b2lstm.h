@@ -119,7 +119,8 @@ int b2_lstm_backward(b2_lstm *layer, const float *weights_dev, const float *x_de
  *   1  persistent kernels, the library chooses the exchange between the blocks of a group (default):
  *      thread-block clusters with transaction barriers in distributed shared memory for as many work
  *      items as fit side by side, the remaining sequences through L2 on the SMs the clusters leave
- *      free; for large batches (many sequences x many units) the tensor-core recurrence of mode 3;
+ *      free; up to 320 units per direction tensor-core kernels with the weights in registers; for large batches (many
+ *      sequences x many units) the tensor-core recurrence of mode 3;
  *   2  persistent kernels, every group as a cluster where a group fits one (128 or 256 units per
  *      direction), through L2 otherwise;
  *   3  tensor-core recurrence (one batched tcgen05 GEMM and one gate kernel per timestep) wherever
@@ -132,7 +133,8 @@ int b2_lstm_backward(b2_lstm *layer, const float *weights_dev, const float *x_de
 int b2_lstm_set_recurrence_mode(b2_lstm *layer, int mode);
 /* Which recurrence kernels the layer's last forward (backward = 0) or backward (backward != 0) sweep really
  * ran, whatever the mode asked for: 0 one launch per timestep, 1 persistent FFMA kernels, 3 tensor-core GEMM
- * and gate kernel per timestep, 5 persistent tensor-core kernels; -1 before the first sweep.  The reference
+ * and gate kernel per timestep, 5 persistent tensor-core kernels, 7 tensor-core kernels with register-resident weights on
+ * thread-block clusters; -1 before the first sweep.  The reference
  * has one code path (layers/LstmLayer.cu:1805-1858), so it has no such query. */
 int b2_lstm_recurrence_path(const b2_lstm *layer, int backward);
 /* Waits for the work enqueued on `stream` and reports what the layer's kernels recorded:

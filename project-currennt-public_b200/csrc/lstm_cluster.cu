@@ -1,17 +1,19 @@
 // Persistent LSTM recurrence for up to 320 units per direction and any number of sequences: ONE launch runs a whole
-// forward (or BPTT) sweep, each thread-block cluster keeps the recurrent weights of one direction in REGISTERS as
-// tensor-core fragments and runs 8, 16 or 32 sequences through all timesteps.
+// forward (or BPTT) sweep; each thread-block cluster keeps the recurrent weights of one direction in REGISTERS as
+// tensor-core fragments and runs a tile of 8 sequences through all timesteps.
 //
 // Replaces the reference's per-timestep loop of 4 cublasSgemm + 1 Thrust functor per direction
 // (layers/LstmLayer.cu:1805-1858,1878-1927 forward with ComputeBlockOutputFn :57-185; :2115-2176,2195-2253 backward with
 // ComputeBlockErrorsFn :237-405 of the reference).
 //
-// What bounds a step.  It is a chain: exchange between the blocks of a cluster (about 500 cycles for the first byte, then
-// about one cycle per 16 bytes received, measured with a probe), recurrent product, cell math.  So the product has to be
-// short for FEW sequences.  tcgen05 with the weights in shared memory costs 40-85 cycles per instruction whatever N is
-// (lstm_ptc.cu); here the weights sit in the registers of the warps that own them, and a warp-level MMA of 16 x 16 weights
-// with 8 sequences takes 8 cycles of its tensor core: 768 cycles per step for 256 units and 8 sequences on 8 SMs, against
-// 2048 cycles of FFMA for the same product.  FFMA wins again at one or two sequences (lstm_persistent.cu).
+// What bounds a step.  It is a chain: exchange between the blocks of a cluster (450 cycles for one 16-byte st.async to be seen by
+// its receiver, then about a cycle per 16 bytes a block receives: measured with probes), recurrent product, cell math.  The
+// product has to be short for FEW sequences.  tcgen05 with the weights in shared memory costs 40-85 cycles per instruction
+// whatever N is (lstm_ptc.cu); here the weights sit in the registers of the warps that own them, and a warp-level MMA of 16 x 16
+// weights with 8 sequences takes 8 cycles of its tensor core: 256 units, 8 sequences on 8 SMs are 768 cycles, against 2048 of FFMA.
+// Measured (B200, us per step forward / backward, against the FFMA kernels of lstm_persistent.cu or, for unit counts those do not
+// have, one launch per step): 256 units per direction, 32 sequences 1.27 / 1.27 (1.74 / 1.56), 4 sequences 0.78 / 1.01 (1.74 / 1.40),
+// 128 sequences 3.6 / 3.8 (6.0 / 5.8); 128 units, 1 sequence 0.66 / 0.81 (1.28 / 0.99); 160 units, 8 sequences 0.95 / 1.0 (20 / 57).
 //
 // Decomposition.  Block b of a cluster of C owns U = 4*WN hidden units with all four gates; its WN warps own 4 units (16 gate
 // rows, one m-tile) each.  Unit counts that do not fill C*U are padded with zero weights; the padding units' outputs are 0.
@@ -20,18 +22,23 @@
 //             exchange by shuffle gives every lane one whole cell.  The lane computes it, and the warp packs its 4 units x 8
 //             sequences as fp16 hi / lo words and stores them into every block's h buffer with st.async (16 bytes each, counted on
 //             a transaction barrier).  No block barrier inside a step.
-//   backward: the block's own gate deltas (4U x sequences, shared memory) times its weight slice transposed give partial
-//             output errors of every unit; each partial goes to the block that owns the unit, which adds the C partials in rank order.
+//   backward: the block's own gate deltas (4U x 8, shared memory) times its weight slice transposed give partial output
+//             errors of every unit; each partial goes to the block that owns the unit, which adds the C partials in a fixed order.
+// Up to 32 units one block does it alone (C = 1): plain shared memory and block barriers take the place of the exchange.
+//
+// Tried and dropped: several tiles per cluster in turn (the second tile costs as much as the first: a warp's own instruction stream,
+// not the exchange, is what fills its time); inputs through a cp.async ring (0.13 us per step more than plain loads).
 //
 // Numerics.  fp32 values enter the tensor cores as two fp16 terms x*S = hi + lo*2^-11 (S a power of two: 2^14 for h, 2^15 for
-// the deltas, which are clipped to [-1, 1], and 2^13 <= max|w|*S < 2^14 per warp tile for the weights), three products, fp32
+// the deltas, which are clipped to [-1, 1], and 2^13 <= max|w|*S < 2^14 per warp for the weights), three products, fp32
 // accumulation, the cross terms (which carry 2^-11) apart: 22 significant bits of each operand, the scheme of the large
-// GEMMs.  The main products run in two chains of at most 10 MMAs.  Activations: expf and a reciprocal refined by one Newton step.
+// GEMMs.  The main products run in two chains of at most 10 MMAs.  Against float64 the outputs and gradients are as close as the
+// FFMA kernels' (relative L2 2.5e-7 / 2.7e-7 against 4.8e-7 / 2.8e-7 at 256 units).
 //
 // Buffers.  A step's h (partial errors) goes into one of two buffers; a warp that sends step t has received all of step t-1,
 // which every warp sent after it had read step t-2, so two buffers need no further hand-shake.  (Backward: the block
 // barrier between the deltas and their product ties the warps of a block together; the deltas have two buffers as well.)
-// Every wait is bounded; on expiry the thread records B2_ERR_STEP_TIMEOUT and all roles leave.  Clusters never wait for each
+// Every wait is bounded; on expiry the thread records B2_ERR_STEP_TIMEOUT and all warps leave.  Clusters never wait for each
 // other, so any number of them may be in flight or queued.
 #include <mutex>
 
@@ -56,22 +63,23 @@ struct ClusterArgs {
     float *y;          // forward: block outputs (written)
     const float *dy;   // backward: output errors (read)
     int *status;
-    int n_items;       // D * ceil(P / (8 * NT))
+    int n_items;       // D * ceil(P / 8): a work item is a tile of 8 sequences of one direction
     int nclusters;
 };
 
-// logistic function with the reference's cut-offs (activation_functions/Logistic.cuh); 1 / d by the hardware approximation and one
-// Newton step (r + r (1 - d r)), which is as exact as the division and has no branches
-__device__ __forceinline__ float cl_logistic(float x) {
-    const float lim = 88.722839f;
-    const float d = 1.0f + expf(fminf(-x, 88.0f));
+// 1 / d, d >= 1: the hardware approximation and one Newton step (r + r (1 - d r)): as exact as the division, without branches
+__device__ __forceinline__ float cl_rcp(float d) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(r, fmaf(-d, r, 1.0f), r);
-    r = x > -lim ? r : 0.0f;
-    return x < lim ? r : 1.0f;
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
-__device__ __forceinline__ float cl_tanh(float x) { return 2.0f * cl_logistic(2.0f * x) - 1.0f; }
+// The exponent limits take the place of the reference's cut-offs (activation_functions/Logistic.cuh): below them the quotients
+// are 0 (logistic) and -1 (tanh).  tanh as (1 - e) / (1 + e), e = exp(-2x), loses less than 2 logistic(2x) - 1 does.
+__device__ __forceinline__ float cl_logistic(float x) { return cl_rcp(1.0f + expf(fminf(-x, 88.0f))); }
+__device__ __forceinline__ float cl_tanh(float x) {
+    const float e = expf(fminf(-2.0f * x, 40.0f));
+    return (1.0f - e) * cl_rcp(1.0f + e);
+}
 
 __device__ __forceinline__ uint32_t split_pair(float x, float S) {   // fp16 hi in the low half, lo in the high half
     const float xs = x * S;
@@ -164,20 +172,39 @@ __device__ __forceinline__ float split_fragments(uint32_t (&f)[N][8]) {
     return inv;
 }
 
+// 4 sequences: columns 0-3 of the 8 an MMA has carry the hi parts, columns 4-7 (lane ^ 2) the lo parts.  m and x are this lane's
+// products with the weights' hi and lo parts; valid in the lanes of columns 0-3
+__device__ __forceinline__ float join_half(float m, float x) {
+    const float cross = __shfl_xor_sync(0xffffffffu, fmaf(x, LO_UNSCALE, m), 2);
+    return fmaf(x + cross, LO_UNSCALE, m);
+}
+
 extern __shared__ __align__(128) unsigned char cl_smem[];
 
 // h and the gate deltas lie in shared memory as [contraction index k][hi of 8 sequences | lo of 8 sequences], 16 bytes each; the two
 // halves change places every other group of 4 rows, so that ldmatrix finds 8 consecutive rows in 8 different bank groups
 __device__ __forceinline__ uint32_t row_off(int k, int half) { return (uint32_t)k * 32u + (uint32_t)((half ^ ((k >> 2) & 1)) * 16); }
 
+// hi and lo of one value into rows of 8 sequences; addr: the tile, plus two bytes per sequence
+__device__ __forceinline__ void st_shared_parts(uint32_t addr, int k, uint32_t parts) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr + row_off(k, 0)), "h"((unsigned short)(parts & 0xffffu)) : "memory");
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr + row_off(k, 1)), "h"((unsigned short)(parts >> 16)) : "memory");
+}
+
 // ---- forward -----------------------------------------------------------------------------------------------------------
-template <int C, int WN, int NT>
+// HALF: at most 4 sequences; columns 0-3 of the tile carry the hi parts, columns 4-7 the lo parts: two MMAs per 16 x 16
+// weights instead of three and half the bytes to exchange
+template <int C, int WN, bool HALF>
+constexpr size_t fwd_smem() { return (size_t)2 * C * 4 * WN * (HALF ? 16 : 32); }
+template <int C, int WN, bool HALF>
 __global__ void __launch_bounds__(32 * WN, 1) lstm_fwd_cluster_kernel(ClusterArgs a) {
     constexpr int U = 4 * WN, KP = C * U, KS = KP / 16;
-    constexpr uint32_t TILE = KP * 32u, BUF = NT * TILE;
+    constexpr uint32_t TILE = KP * (HALF ? 16u : 32u);
     __shared__ __align__(8) unsigned long long bars[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int uu = lane >> 3, n = 2 * tig + (g & 1);     // the cell this lane computes: unit uu of the warp's four, sequence n
+    // the cell this lane computes: unit uu of the warp's four, sequence n (HALF: the lanes with tig < 2)
+    const int uu = lane >> 3, n = 2 * (HALF ? tig & 1 : tig) + (g & 1);
+    const bool owner = !HALF || tig < 2;
     const uint32_t rank = cluster_ctarank(), hbuf = smem_u32(cl_smem);
     const int P = a.sh.P, T = a.sh.T, ls = a.sh.ls, els = a.sh.els, D = a.sh.D;
     const LstmOffsets off = lstm_offsets(a.sh.pls, ls, els);
@@ -188,15 +215,25 @@ __global__ void __launch_bounds__(32 * WN, 1) lstm_fwd_cluster_kernel(ClusterArg
         mbar_init(bar(1), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    cluster_sync_all();   // a peer's shared memory may be touched only once the peer runs
+    if constexpr (C > 1) cluster_sync_all();   // a peer's shared memory may be touched only once the peer runs
+    else __syncthreads();
+
+    // peers this lane sends to: C / PEERS of them (shared-memory addresses of a peer are linear)
+    constexpr int PEERS = HALF ? 8 : 4, NP = C > 1 ? (C + PEERS - 1) / PEERS : 1;
+    uint32_t peer[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) peer[q] = C > 1 ? map_to_rank(hbuf, (uint32_t)((HALF ? lane >> 2 : lane >> 3) + PEERS * q) & (C - 1)) : hbuf;
 
     uint32_t wf[KS][8];
     float inv = 1.0f;
     int cur_d = -1;
     unsigned ev = 0;      // steps published so far
     bool ok = true;
+    // ldmatrix rows of this lane: hi and lo of one k-step, or (HALF) two k-steps
+    const uint32_t ldsm_lane = HALF ? (uint32_t)lane * 16u
+        : (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)) * 32u + (uint32_t)(((lane >> 4) ^ ((lane >> 2) & 1)) * 16);
     for (int item = (int)(blockIdx.x / C); item < a.n_items && ok; item += a.nclusters) {
-        const int d = item % D, p0 = (item / D) * 8 * NT;
+        const int d = item % D, pg = (item / D) * 8 + n;
         if (d != cur_d) {
             // row r of the tile: unit r/2 mod 4, gate (r mod 2) + 2 * (r / 8), so that rows g and g + 8 are two gates of one unit
             const int jw = (int)rank * U + warp * 4 + (g >> 1);
@@ -220,137 +257,144 @@ __global__ void __launch_bounds__(32 * WN, 1) lstm_fwd_cluster_kernel(ClusterArg
 #pragma unroll
             for (int q = 0; q < 3; ++q) pw[q] = __ldg(a.w + off.peep + (size_t)q * ls + u);
         }
-        int len[NT], Tc = 0;
-        float cprev[NT], pre_n[NT][4];
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            len[i] = sequence_length(a, p0 + 8 * i + n);
-            Tc = max(Tc, len[i]);
-            cprev[i] = 0.0f;
-        }
-        Tc = warp_max(Tc);    // the cluster's longest sequence: beyond it all frames are padding
-        // what a step reads from HBM is independent of the recurrence and is fetched one step ahead
+        const int len = sequence_length(a, pg), Tc = warp_max(len);   // beyond the tile's longest sequence all frames are padding
+        const bool unit = j < els, mine = unit && pg < P && owner;
+        // Frame t of this lane's cell: uniform base of the frame's row plus 32-bit offsets that stay the same.  Loads are
+        // unconditional (a value behind a branch would have to arrive before the branches join): cells that do not exist read
+        // the offsets of one that does.
+        const size_t row0 = (size_t)((item / D) * 8);
+        const uint32_t nc = (uint32_t)(pg < P ? n : 0), uc = (uint32_t)(d * els + (unit ? j : 0));
+        const uint32_t of_y = (nc * ls + uc) * 4u, of_a = (nc * 4u * ls + uc) * 4u, of_g = (uint32_t)ls * 4u;
+        float cp = 0.0f, pre[4];
+        // pre-activations are independent of the recurrence and fetched a step ahead, BEFORE the step waits for its peers: behind
+        // the step's stores the same loads cost 0.2 us per step
         auto fetch = [&](int s) {
-            const int t = d ? Tc - 1 - s : s;
+            const int sc = s < Tc ? s : Tc - 1, t = d ? Tc - 1 - sc : sc;
+            const char *ap = reinterpret_cast<const char *>(a.bf.acts + ((size_t)t * P + row0) * 4 * ls);
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) pre_n[i][q] = 0.0f;
-                if (t < len[i] && j < els) {
-                    const float *ap = a.bf.acts + ((size_t)t * P + p0 + 8 * i + n) * 4 * ls + u;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) pre_n[i][q] = ap[(size_t)q * ls];
-                }
-            }
+            for (int q = 0; q < 4; ++q) pre[q] = *reinterpret_cast<const float *>(ap + (of_a + (uint32_t)q * of_g));
         };
-        const uint32_t ldsm_lane = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)) * 32u + (uint32_t)(((lane >> 4) ^ ((lane >> 2) & 1)) * 16);
-        if (Tc > 0) fetch(0);
-        for (int s = 0; s < Tc; ++s) {
-            const int t = d ? Tc - 1 - s : s;
-            const bool publish = s + 1 < Tc;
-            float x[NT][4];
+        auto step = [&](int s) {
+                const int t = d ? Tc - 1 - s : s;
+                const bool publish = s + 1 < Tc, real = t < len && unit;
+                if (C > 1 && publish && threadIdx.x == 0) mbar_expect_tx(bar(ev), TILE);
+                float x[4];
 #pragma unroll
-            for (int i = 0; i < NT; ++i)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) x[i][q] = pre_n[i][q] + b4[q];
-            if (s + 1 < Tc) fetch(s + 1);
-            if (publish && threadIdx.x == 0) mbar_expect_tx(bar(ev), BUF);
-            if (s > 0) {
-                ok = __all_sync(0xffffffffu, wait_bounded(bar(ev - 1), ((ev - 1) >> 1) & 1u, a.status));
-                if (!ok) break;
-                const uint32_t hb = hbuf + ((ev - 1) & 1u) * BUF + ldsm_lane;
-#pragma unroll
-                for (int i = 0; i < NT; ++i) {
-                    float m0[4] = {0, 0, 0, 0}, m1[4] = {0, 0, 0, 0}, xa[4] = {0, 0, 0, 0}, xb[4] = {0, 0, 0, 0};
-#pragma unroll
-                    for (int ks = 0; ks < KS; ++ks) {
-                        uint32_t b[4];
-                        ldsm_x4_t(b, hb + (uint32_t)i * TILE + (uint32_t)ks * 512u);
-                        const uint32_t *f = wf[ks];
-                        mma16816(xa, f[4], f[5], f[6], f[7], b[0], b[1]);
-                        mma16816((ks & 1) ? m1 : m0, f[0], f[1], f[2], f[3], b[0], b[1]);
-                        mma16816(xb, f[0], f[1], f[2], f[3], b[2], b[3]);
+                for (int q = 0; q < 4; ++q) x[q] = pre[q] + b4[q];
+                fetch(s + 1);
+                if (s > 0) {
+                    if constexpr (C > 1) {
+                        ok = __all_sync(0xffffffffu, wait_bounded(bar(ev - 1), ((ev - 1) >> 1) & 1u, a.status));
+                        if (!ok) return;
+                    } else {
+                        __syncthreads();
                     }
+                    const uint32_t hb = hbuf + ((ev - 1) & 1u) * TILE + ldsm_lane;
+                    float m0[4] = {0, 0, 0, 0}, m1[4] = {0, 0, 0, 0}, xa[4] = {0, 0, 0, 0}, xb[4] = {0, 0, 0, 0};
                     float z[4];
+                    if constexpr (HALF) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) z[e] = ((m0[e] + m1[e]) + (xa[e] + xb[e]) * LO_UNSCALE) * inv;
+                        for (int ks = 0; ks < KS; ks += 2) {
+                            uint32_t b[4];
+                            ldsm_x4_t(b, hb + (uint32_t)ks * 256u);
+                            mma16816(m0, wf[ks][0], wf[ks][1], wf[ks][2], wf[ks][3], b[0], b[1]);
+                            mma16816(xa, wf[ks][4], wf[ks][5], wf[ks][6], wf[ks][7], b[0], b[1]);
+                            mma16816(m1, wf[ks + 1][0], wf[ks + 1][1], wf[ks + 1][2], wf[ks + 1][3], b[2], b[3]);
+                            mma16816(xb, wf[ks + 1][4], wf[ks + 1][5], wf[ks + 1][6], wf[ks + 1][7], b[2], b[3]);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) z[e] = join_half(m0[e] + m1[e], xa[e] + xb[e]) * inv;
+                    } else {
+#pragma unroll
+                        for (int ks = 0; ks < KS; ++ks) {
+                            uint32_t b[4];
+                            ldsm_x4_t(b, hb + (uint32_t)ks * 512u);
+                            const uint32_t *f = wf[ks];
+                            mma16816(xa, f[4], f[5], f[6], f[7], b[0], b[1]);
+                            mma16816((ks & 1) ? m1 : m0, f[0], f[1], f[2], f[3], b[0], b[1]);
+                            mma16816(xb, f[0], f[1], f[2], f[3], b[2], b[3]);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) z[e] = ((m0[e] + m1[e]) + (xa[e] + xb[e]) * LO_UNSCALE) * inv;
+                    }
                     // lanes with even g hold gates 0 and 2 of columns 2 tig and 2 tig + 1, their partners (lane ^ 4) gates 1 and 3
                     const bool odd = g & 1;
                     const float r0 = __shfl_xor_sync(0xffffffffu, odd ? z[0] : z[1], 4);
                     const float r1 = __shfl_xor_sync(0xffffffffu, odd ? z[2] : z[3], 4);
-                    x[i][0] += odd ? r0 : z[0];
-                    x[i][1] += odd ? z[1] : r0;
-                    x[i][2] += odd ? r1 : z[2];
-                    x[i][3] += odd ? z[3] : r1;
+                    x[0] += odd ? r0 : z[0];
+                    x[1] += odd ? z[1] : r0;
+                    x[2] += odd ? r1 : z[2];
+                    x[3] += odd ? z[3] : r1;
                 }
-            }
-            float ni[NT], ig[NT], fg[NT], og[NT], hh[NT];
+                float ni = cl_tanh(x[0]), ig = cl_logistic(x[1] + cp * pw[0]), fg = cl_logistic(x[2] + cp * pw[1]);
+                float c = ni * ig + cp * fg;
+                float og = cl_logistic(x[3] + c * pw[2]);
+                float hh = cl_tanh(c) * og;
+                if (!real) { ni = ig = fg = og = hh = c = 0.0f; }   // padding frame or unit
+                if (publish) {
+                    const uint32_t v = split_pair(hh, S_H);
+                    const uint32_t hd = hbuf + (ev & 1u) * TILE;
+                    if constexpr (C > 1) {
+                        // chunks of 16 bytes: hi or lo of 8 sequences of a unit (HALF: hi and lo of 4)
+                        const int ch = HALF ? lane & 3 : lane & 7, kk = (int)rank * U + warp * 4 + (HALF ? ch : ch >> 1);
+                        const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 4);
+                        const uint32_t word = (g & 1) ? ((o >> 16) | (v & 0xffff0000u)) : ((v & 0xffffu) | (o << 16));
+                        uint32_t q4[4];
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                const float cp = cprev[i];
-                ni[i] = cl_tanh(x[i][0]);
-                ig[i] = cl_logistic(x[i][1] + cp * pw[0]);
-                fg[i] = cl_logistic(x[i][2] + cp * pw[1]);
-                float c = ni[i] * ig[i] + cp * fg[i];
-                og[i] = cl_logistic(x[i][3] + c * pw[2]);
-                hh[i] = cl_tanh(c) * og[i];
-                if (!(t < len[i] && j < els)) { ni[i] = ig[i] = fg[i] = og[i] = hh[i] = c = 0.0f; }   // padding frame or unit
-                cprev[i] = c;
-            }
-            if (publish) {
-                const int ch = lane & 7;     // chunk of 16 bytes: unit ch / 2 of the warp, hi or lo
-                const int kk = (int)rank * U + warp * 4 + (ch >> 1);
+                        for (int q = 0; q < 4; ++q)
+                            q4[q] = __shfl_sync(0xffffffffu, word, HALF ? 8 * ch + (q & 1) + 4 * (q >> 1) : 4 * ch + q);
+                        const uint32_t o2 = hd - hbuf + (HALF ? (uint32_t)kk * 16u : row_off(kk, ch & 1));
 #pragma unroll
-                for (int i = 0; i < NT; ++i) {
-                    const uint32_t v = split_pair(hh[i], S_H);
-                    const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 4);
-                    const uint32_t word = (g & 1) ? ((o >> 16) | (v & 0xffff0000u)) : ((v & 0xffffu) | (o << 16));
-                    uint32_t q4[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) q4[q] = __shfl_sync(0xffffffffu, word, 4 * ch + q);
-                    const uint32_t la = hbuf + (ev & 1u) * BUF + (uint32_t)i * TILE + row_off(kk, ch & 1);
-#pragma unroll
-                    for (int r4 = 0; r4 < C / 4; ++r4) {
-                        const uint32_t r = (uint32_t)(lane >> 3) + 4u * r4;
-                        st_async_v4(map_to_rank(la, r), q4[0], q4[1], q4[2], q4[3], map_to_rank(bar(ev), r));
+                        for (int q = 0; q < NP; ++q)
+                            if (C % PEERS == 0 || (lane >> 2) < C) st_async_v4(peer[q] + o2, q4[0], q4[1], q4[2], q4[3], peer[q] + (bar(ev) - hbuf));
+                    } else {
+                        st_shared_parts(hd + 2u * (uint32_t)n, warp * 4 + uu, v);
                     }
                 }
-                ++ev;
-            }
-            // the peers are waiting for h: the layer's own state goes to memory after it is on its way
-#pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                const int pg = p0 + 8 * i + n;
-                if (pg < P && j < els) {
-                    const size_t f = (size_t)t * P + pg;
-                    float *ap = a.bf.acts + f * 4 * ls + u;
-                    ap[0] = ni[i]; ap[ls] = ig[i]; ap[2 * (size_t)ls] = fg[i]; ap[3 * (size_t)ls] = og[i];
-                    a.bf.cells[f * ls + u] = cprev[i];
-                    a.y[f * ls + u] = hh[i];
+                if (publish) ++ev;
+                cp = c;
+                // the peers are waiting for h: the layer's own state goes to memory after it is on its way
+                if (mine) {
+                    char *ap = reinterpret_cast<char *>(a.bf.acts + ((size_t)t * P + row0) * 4 * ls);
+                    *reinterpret_cast<float *>(ap + of_a) = ni;
+                    *reinterpret_cast<float *>(ap + (of_a + of_g)) = ig;
+                    *reinterpret_cast<float *>(ap + (of_a + 2u * of_g)) = fg;
+                    *reinterpret_cast<float *>(ap + (of_a + 3u * of_g)) = og;
+                    const size_t r = ((size_t)t * P + row0) * ls;
+                    *reinterpret_cast<float *>(reinterpret_cast<char *>(a.bf.cells + r) + of_y) = c;
+                    *reinterpret_cast<float *>(reinterpret_cast<char *>(a.y + r) + of_y) = hh;
                 }
+        };
+        if (Tc > 0) fetch(0);
+#pragma unroll 1
+        for (int s = 0; s < Tc && ok; ++s) step(s);
+        // frames beyond the tile's longest sequence
+        if (mine)
+            for (int t = Tc; t < T; ++t) {
+                const size_t f = ((size_t)t * P + pg) * ls + u;
+                a.y[f] = 0.0f;
+                a.bf.cells[f] = 0.0f;
             }
-        }
-        // frames beyond the cluster's longest sequence
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            const int pg = p0 + 8 * i + n;
-            if (pg < P && j < els)
-                for (int t = Tc; t < T; ++t) {
-                    const size_t f = ((size_t)t * P + pg) * ls + u;
-                    a.y[f] = 0.0f;
-                    a.bf.cells[f] = 0.0f;
-                }
-        }
+        if (C == 1) __syncthreads();
     }
-    cluster_sync_all();   // nobody leaves while a peer may still write into its shared memory
+    if constexpr (C > 1) cluster_sync_all();   // nobody leaves while a peer may still write into its shared memory
 }
 
 // ---- backward ------------------------------------------------------------------------------------------------------------
-template <int C, int WN, int NT>
+// a warp: MT m-tiles of 16 source units times the block's NK k-steps of gate rows.  One block alone: one m-tile per four warps,
+// which take a quarter of the rows each and stand for the source blocks of a cluster of four
+template <int C, int WN>
+struct BwdGeo {
+    static constexpr int U = 4 * WN, MT = C > 1 ? C / 4 : 1, NK = C > 1 ? WN : WN / 4, SRC = C > 1 ? C : 4;
+    static constexpr uint32_t BUF = SRC * U * 32u;          // partial errors: [source][unit][8 floats]
+    static constexpr uint32_t DTILE = 4u * U * 32u;         // the block's own deltas
+    static constexpr size_t smem() { return (size_t)2 * (BUF + DTILE); }
+};
+template <int C, int WN>
 __global__ void __launch_bounds__(32 * WN, 1) lstm_bwd_cluster_kernel(ClusterArgs a) {
-    constexpr int U = 4 * WN, KP = C * U, MT = C / 4;     // MT m-tiles of 16 source units per warp
-    constexpr uint32_t BUF = KP * 32u * NT;               // partial errors received per step: [source block][unit][8 * NT floats]
-    constexpr uint32_t DTILE = 4u * U * 32u;              // the block's own deltas of 8 sequences
+    typedef BwdGeo<C, WN> G;
+    constexpr int U = G::U, MT = G::MT, NK = G::NK, SRC = G::SRC;
+    constexpr uint32_t BUF = G::BUF, DTILE = G::DTILE;
     __shared__ __align__(8) unsigned long long bars[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int uu = lane >> 3, n = 2 * tig + (g & 1);
@@ -364,30 +408,43 @@ __global__ void __launch_bounds__(32 * WN, 1) lstm_bwd_cluster_kernel(ClusterArg
         mbar_init(bar(1), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    cluster_sync_all();
+    if constexpr (C > 1) cluster_sync_all();
+    else __syncthreads();
+    const int tile0 = C > 1 ? warp * MT : warp >> 2, k0 = C > 1 ? 0 : (warp & 3) * NK;   // first m-tile and k-step of this warp
+    const uint32_t ldsm_lane = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)) * 32u + (uint32_t)(((lane >> 4) ^ ((lane >> 2) & 1)) * 16) +
+                               (uint32_t)k0 * 512u;
 
-    uint32_t wf[MT * WN][8];
+    // lane's source unit of m-tile mt (even tig row g, odd tig row g + 8): the block that owns it, its place there
+    uint32_t peer[MT], place[MT];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        const int src = (tile0 + mt) * 16 + g + ((tig & 1) ? 8 : 0);
+        peer[mt] = C > 1 ? map_to_rank(ebuf, (uint32_t)(src / U)) : ebuf;
+        place[mt] = (((C > 1 ? rank : (uint32_t)(warp & 3)) * U + (uint32_t)(src % U)) * 8u + 4u * (uint32_t)(tig >> 1)) * 4u;
+    }
+
+    uint32_t wf[MT * NK][8];
     float inv = 1.0f;
     int cur_d = -1;
     unsigned ev = 0;
     bool ok = true;
     for (int item = (int)(blockIdx.x / C); item < a.n_items && ok; item += a.nclusters) {
-        const int d = item % D, p0 = (item / D) * 8 * NT;
+        const int d = item % D, pg = (item / D) * 8 + n;
         if (d != cur_d) {
             // rows: source units; contraction index 16 ks + 4 gate + unit: the block's own gate rows
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int ks = 0; ks < WN; ++ks)
+                for (int ks = 0; ks < NK; ++ks)
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        const int src = (warp * MT + mt) * 16 + g + ((e & 2) ? 8 : 0);
+                        const int src = (tile0 + mt) * 16 + g + ((e & 2) ? 8 : 0);
                         const int pos = 2 * tig + (e & 1) + ((e & 4) ? 8 : 0);
-                        const int jw = (int)rank * U + ks * 4 + (pos & 3);
-                        wf[mt * WN + ks][e] = (jw < els && src < els)
+                        const int jw = (int)rank * U + (k0 + ks) * 4 + (pos & 3);
+                        wf[mt * NK + ks][e] = (jw < els && src < els)
                             ? __float_as_uint(__ldg(a.w + off.rec + ((size_t)(pos >> 2) * ls + (size_t)d * els + jw) * els + src)) : 0u;
                     }
-            inv = split_fragments<MT * WN>(wf) * (1.0f / S_D);
+            inv = split_fragments<MT * NK>(wf) * (1.0f / S_D);
             cur_d = d;
         }
         const int u = d * els + j;
@@ -395,108 +452,75 @@ __global__ void __launch_bounds__(32 * WN, 1) lstm_bwd_cluster_kernel(ClusterArg
         if (j < els)
 #pragma unroll
             for (int q = 0; q < 3; ++q) pw[q] = __ldg(a.w + off.peep + (size_t)q * ls + u);
-        int len[NT], Tc = 0;
-        float st_ce[NT], st_dig[NT], st_dfg[NT], st_fg[NT], cc[NT];   // values of the step before; the cell state of this one
-        float e_n[NT], a4_n[NT][4], cp_n[NT];
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            len[i] = sequence_length(a, p0 + 8 * i + n);
-            Tc = max(Tc, len[i]);
-            st_ce[i] = st_dig[i] = st_dfg[i] = st_fg[i] = cc[i] = 0.0f;
-        }
-        Tc = warp_max(Tc);
-        auto fetch = [&](int s) {
-            const int t = d ? s : Tc - 1 - s, prev = d ? t + 1 : t - 1;
-#pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                const int pg = p0 + 8 * i + n;
-                e_n[i] = cp_n[i] = 0.0f;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) a4_n[i][q] = 0.0f;
-                if (j < els && pg < P) {
-                    const size_t f = (size_t)t * P + pg;
-                    if (t < len[i]) {
-                        e_n[i] = a.dy[f * ls + u];
-                        const float *ap = a.bf.acts + f * 4 * ls + u;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) a4_n[i][q] = ap[(size_t)q * ls];
-                        if (s == 0) cc[i] = a.bf.cells[f * ls + u];
-                    }
-                    if (s != Tc - 1) cp_n[i] = a.bf.cells[((size_t)prev * P + pg) * ls + u];
-                }
-            }
+        const int len = sequence_length(a, pg), Tc = warp_max(len);
+        const bool unit = j < els, mine = unit && pg < P;
+        const size_t row0 = (size_t)((item / D) * 8);      // addresses as in the forward kernel
+        const uint32_t nc = (uint32_t)(pg < P ? n : 0), uc = (uint32_t)(d * els + (unit ? j : 0));
+        const uint32_t of_y = (nc * ls + uc) * 4u, of_a = (nc * 4u * ls + uc) * 4u, of_g = (uint32_t)ls * 4u;
+        struct In { float e, ni, ig, fg, og, cp; };     // output error, activations, the previous frame's cell state
+        In in = {0, 0, 0, 0, 0, 0};
+        float cc = 0.0f, st_fg = 0.0f, st_ce = 0.0f, st_dig = 0.0f, st_dfg = 0.0f;   // this frame's cell state; values of the step before
+        auto fetch = [&](int s) {      // a step ahead, before the wait (see the forward kernel)
+            const int sc = s < Tc ? s : Tc - 1, t = d ? sc : Tc - 1 - sc, prev = sc == Tc - 1 ? t : (d ? t + 1 : t - 1);
+            in.e = *reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.dy + ((size_t)t * P + row0) * ls) + of_y);
+            const char *ap = reinterpret_cast<const char *>(a.bf.acts + ((size_t)t * P + row0) * 4 * ls);
+            in.ni = *reinterpret_cast<const float *>(ap + of_a);
+            in.ig = *reinterpret_cast<const float *>(ap + (of_a + of_g));
+            in.fg = *reinterpret_cast<const float *>(ap + (of_a + 2u * of_g));
+            in.og = *reinterpret_cast<const float *>(ap + (of_a + 3u * of_g));
+            in.cp = *reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.bf.cells + ((size_t)prev * P + row0) * ls) + of_y);
         };
-        const uint32_t ldsm_lane = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)) * 32u + (uint32_t)(((lane >> 4) ^ ((lane >> 2) & 1)) * 16);
-        if (Tc > 0) fetch(0);
-        for (int s = 0; s < Tc; ++s) {
-            const int t = d ? s : Tc - 1 - s;
-            const bool first = (s == 0), last = (s == Tc - 1);
-            float e[NT], a4[NT][4], cp[NT], dd[NT][4];
-#pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                e[i] = e_n[i];
-                cp[i] = cp_n[i];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) a4[i][q] = a4_n[i][q];
-            }
-            if (!last) fetch(s + 1);
-            if (!last && threadIdx.x == 0) mbar_expect_tx(bar(ev), BUF);
-            if (!first) {
-                ok = wait_bounded(bar(ev - 1), ((ev - 1) >> 1) & 1u, a.status);
-                const float *pe = reinterpret_cast<const float *>(cl_smem + ((ev - 1) & 1u) * BUF) + (size_t)(warp * 4 + uu) * NT * 8 + n;
-#pragma unroll
-                for (int i = 0; i < NT; ++i) {
+        auto step = [&](int s) {
+                const int t = d ? s : Tc - 1 - s;
+                const bool first = (s == 0), last = (s == Tc - 1), real = t < len && unit;
+                if (C > 1 && !last && threadIdx.x == 0) mbar_expect_tx(bar(ev), BUF);
+                float e = in.e;
+                const float nig = in.ni, ig = in.ig, fg = in.fg, og = in.og, cp = last || !mine ? 0.0f : in.cp;    // no previous cell state at the last step
+                // ComputeBlockErrorsFn, the part that does not wait for the peers' partial errors: with e the output error,
+                //   dog = k_og e, ce = k_ce e + p_og dog + carry, d{ni,ig,fg} = k_{ni,ig,fg} ce
+                const float tc = cl_tanh(cc);
+                const float k_og = d_logistic(og) * tc, k_ce = og * d_tanh(tc);
+                const float carry = st_fg * st_ce + pw[0] * st_dig + pw[1] * st_dfg;      // zeros at the first step
+                const float k_ni = ig * d_tanh(nig), k_ig = d_logistic(ig) * nig, k_fg = d_logistic(fg) * cp;
+                fetch(s + 1);
+                if (!first) {
+                    if constexpr (C > 1) ok = wait_bounded(bar(ev - 1), ((ev - 1) >> 1) & 1u, a.status);
+                    else __syncthreads();
+                    const float *pe = reinterpret_cast<const float *>(cl_smem + ((ev - 1) & 1u) * BUF) + (warp * 4 + uu) * 8 + n;
+                    // rank order; four chains where there are more than four sources
                     float sum = 0.0f;
+                    if constexpr (SRC > 4) {
+                        float s4[4] = {0, 0, 0, 0};
 #pragma unroll
-                    for (int src = 0; src < C; ++src) sum += pe[(src * U * NT + i) * 8];
-                    e[i] += sum;
-                }
-            }
+                        for (int src = 0; src < SRC; ++src) s4[src & 3] += pe[src * U * 8];
+                        sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+                    } else {
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                const float nig = a4[i][0], ig = a4[i][1], fg = a4[i][2], og = a4[i][3];
-                const float tc = cl_tanh(cc[i]);
-                float dog = d_logistic(og) * tc * e[i];
-                float ce = og * d_tanh(tc) * e[i] + pw[2] * dog;
-                ce += st_fg[i] * st_ce[i] + pw[0] * st_dig[i] + pw[1] * st_dfg[i];    // zeros at the first step
-                float dni = limited_error(ig * d_tanh(nig) * ce);
-                float dfg = limited_error(d_logistic(fg) * cp[i] * ce);               // no previous cell state at the last step: cp = 0
-                float dig = limited_error(d_logistic(ig) * nig * ce);
-                dog = limited_error(dog);
-                const bool real = t < len[i] && j < els;
-                st_fg[i] = real ? fg : 0.0f;
-                st_ce[i] = real ? ce : 0.0f;
-                dd[i][0] = real ? dni : 0.0f; dd[i][1] = st_dig[i] = real ? dig : 0.0f;
-                dd[i][2] = st_dfg[i] = real ? dfg : 0.0f; dd[i][3] = real ? dog : 0.0f;
-                cc[i] = cp[i];          // the previous step's cell state is the next one's own
-            }
-            if (!last) {
-#pragma unroll
-                for (int i = 0; i < NT; ++i)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t v = split_pair(dd[i][q], S_D);
-                        const int k = warp * 16 + q * 4 + uu;
-                        const uint32_t o = dbuf + ((ev & 1u) * NT + (uint32_t)i) * DTILE + 2u * (uint32_t)n;
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(o + row_off(k, 0)), "h"((unsigned short)(v & 0xffffu)) : "memory");
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(o + row_off(k, 1)), "h"((unsigned short)(v >> 16)) : "memory");
+                        for (int src = 0; src < SRC; ++src) sum += pe[src * U * 8];
                     }
-                ok = !__syncthreads_or(!ok);
-                if (!ok) break;
-#pragma unroll 1
-                for (int i = 0; i < NT; ++i) {
+                    e += sum;
+                }
+                const float dog_ = k_og * e;
+                float ce = __fadd_rn(__fadd_rn(__fmul_rn(k_ce, e), __fmul_rn(pw[2], dog_)), carry);   // rounded term by term, as on the host
+                float dd[4] = {limited_error(k_ni * ce), limited_error(k_ig * ce), limited_error(k_fg * ce), limited_error(dog_)};
+                if (!real) ce = dd[0] = dd[1] = dd[2] = dd[3] = 0.0f;
+                if (!last) {
+                    const uint32_t db = dbuf + (ev & 1u) * DTILE;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) st_shared_parts(db + 2u * (uint32_t)n, warp * 16 + q * 4 + uu, split_pair(dd[q], S_D));
+                    if (__syncthreads_or(!ok)) { ok = false; return; }
                     float m0[MT][4], xa[MT][4];
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
                         for (int q = 0; q < 4; ++q) m0[mt][q] = xa[mt][q] = 0.0f;
 #pragma unroll
-                    for (int ks = 0; ks < WN; ++ks) {
+                    for (int ks = 0; ks < NK; ++ks) {
                         uint32_t b[4];
-                        ldsm_x4_t(b, dbuf + ((ev & 1u) * NT + (uint32_t)i) * DTILE + ldsm_lane + (uint32_t)ks * 512u);
+                        ldsm_x4_t(b, db + ldsm_lane + (uint32_t)ks * 512u);
 #pragma unroll
                         for (int mt = 0; mt < MT; ++mt) {
-                            const uint32_t *f = wf[mt * WN + ks];
+                            const uint32_t *f = wf[mt * NK + ks];
                             mma16816(xa[mt], f[4], f[5], f[6], f[7], b[0], b[1]);
                             mma16816(m0[mt], f[0], f[1], f[2], f[3], b[0], b[1]);
                             mma16816(xa[mt], f[0], f[1], f[2], f[3], b[2], b[3]);
@@ -511,138 +535,157 @@ __global__ void __launch_bounds__(32 * WN, 1) lstm_bwd_cluster_kernel(ClusterArg
                         const bool odd = tig & 1;
                         const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1);
                         const float r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
-                        const int src = (warp * MT + mt) * 16 + g + (odd ? 8 : 0);
-                        const uint32_t owner = (uint32_t)(src / U), ul = (uint32_t)(src % U);
-                        const uint32_t la = ebuf + (ev & 1u) * BUF + (((rank * U + ul) * NT + (uint32_t)i) * 8u + 4u * (uint32_t)(tig >> 1)) * 4u;
-                        if (odd)
-                            st_async_v4(map_to_rank(la, owner), __float_as_uint(r0), __float_as_uint(r1), __float_as_uint(v[2]),
-                                        __float_as_uint(v[3]), map_to_rank(bar(ev), owner));
+                        const float4 f4 = make_float4(odd ? r0 : v[0], odd ? r1 : v[1], odd ? v[2] : r0, odd ? v[3] : r1);
+                        const uint32_t o2 = (ev & 1u) * BUF + place[mt];
+                        if constexpr (C > 1)
+                            st_async_v4(peer[mt] + o2, __float_as_uint(f4.x), __float_as_uint(f4.y), __float_as_uint(f4.z), __float_as_uint(f4.w),
+                                        peer[mt] + (bar(ev) - ebuf));
                         else
-                            st_async_v4(map_to_rank(la, owner), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(r0),
-                                        __float_as_uint(r1), map_to_rank(bar(ev), owner));
+                            *reinterpret_cast<float4 *>(cl_smem + o2) = f4;
                     }
                 }
-                ++ev;
-            }
-            // the deltas go to memory after the partial errors the peers wait for have been sent
+                if (!last) ++ev;
+                cc = cp;                // the previous frame's cell state is the next step's own
+                st_fg = real ? fg : 0.0f; st_ce = ce; st_dig = dd[1]; st_dfg = dd[2];
+                // the deltas go to memory after the partial errors the peers wait for have been sent
+                if (mine) {
+                    char *dl = reinterpret_cast<char *>(a.bf.deltas + ((size_t)t * P + row0) * 4 * ls);
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                const int pg = p0 + 8 * i + n;
-                if (pg < P && j < els) {
-                    float *dl = a.bf.deltas + ((size_t)t * P + pg) * 4 * ls + u;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) dl[(size_t)q * ls] = dd[i][q];
+                    for (int q = 0; q < 4; ++q) *reinterpret_cast<float *>(dl + (of_a + (uint32_t)q * of_g)) = dd[q];
                 }
-            }
+        };
+        if (Tc > 0 && mine) {
+            const int t = d ? 0 : Tc - 1;
+            if (t < len) cc = a.bf.cells[((size_t)t * P + pg) * ls + u];
         }
+        if (Tc > 0) fetch(0);
+#pragma unroll 1
+        for (int s = 0; s < Tc && ok; ++s) step(s);
         ok = !__syncthreads_or(!ok);
+        if (mine)
+            for (int t = Tc; t < T; ++t) {
+                float *dl = a.bf.deltas + ((size_t)t * P + pg) * 4 * ls + u;
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            const int pg = p0 + 8 * i + n;
-            if (pg < P && j < els)
-                for (int t = Tc; t < T; ++t) {
-                    float *dl = a.bf.deltas + ((size_t)t * P + pg) * 4 * ls + u;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) dl[(size_t)q * ls] = 0.0f;
-                }
-        }
+                for (int q = 0; q < 4; ++q) dl[(size_t)q * ls] = 0.0f;
+            }
     }
-    cluster_sync_all();
+    if constexpr (C > 1) cluster_sync_all();
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------
 typedef void (*Kernel)(ClusterArgs);
-struct Variant { int C, WN, NT; Kernel fwd, bwd; };
-template <int C, int WN, int NT>
-constexpr Variant variant() { return Variant{C, WN, NT, lstm_fwd_cluster_kernel<C, WN, NT>, lstm_bwd_cluster_kernel<C, WN, NT>}; }
-#define VARIANTS_OF(C, WN) variant<C, WN, 1>(), variant<C, WN, 2>(), variant<C, WN, 4>()
-const Variant VARIANTS[] = {VARIANTS_OF(4, 2), VARIANTS_OF(4, 4), VARIANTS_OF(4, 6), VARIANTS_OF(4, 8), VARIANTS_OF(8, 4), VARIANTS_OF(8, 5),
-                            VARIANTS_OF(8, 6), VARIANTS_OF(8, 7), VARIANTS_OF(8, 8), VARIANTS_OF(16, 2), VARIANTS_OF(16, 4),
-                            variant<16, 5, 1>(), variant<16, 5, 2>()};
-constexpr int NVARIANTS = (int)(sizeof(VARIANTS) / sizeof(VARIANTS[0]));
-
-size_t smem_bytes(const Variant &v, bool backward) {
-    const size_t buf = (size_t)v.C * 4 * v.WN * 32 * v.NT;
-    return 2 * buf + (backward ? (size_t)2 * v.NT * 16 * v.WN * 32 : 0);
+struct Variant {
+    int C, WN;
+    bool half;
+    Kernel kern;
+    size_t smem;
+};
+template <int C, int WN, bool HALF>
+constexpr Variant fwd_variant() {
+    return Variant{C, WN, HALF, lstm_fwd_cluster_kernel<C, WN, HALF>, fwd_smem<C, WN, HALF>()};
 }
+template <int C, int WN>
+constexpr Variant bwd_variant() {
+    return Variant{C, WN, false, lstm_bwd_cluster_kernel<C, WN>, BwdGeo<C, WN>::smem()};
+}
+#define SHAPES(X) X(1, 4) X(1, 8) X(4, 4) X(4, 6) X(4, 8) X(8, 4) X(8, 5) X(8, 6) X(8, 7) X(8, 8) X(16, 2) X(16, 4) X(16, 5)
+#define SHAPES_HALF(X) X(4, 4) X(4, 6) X(4, 8) X(8, 4) X(8, 5) X(8, 6) X(8, 7) X(8, 8) X(16, 2) X(16, 4) X(16, 5)
+#define FWD_FULL(C, WN) fwd_variant<C, WN, false>(),
+#define FWD_HALF(C, WN) fwd_variant<C, WN, true>(),
+#define BWD_FULL(C, WN) bwd_variant<C, WN>(),
+const Variant FWD[] = {SHAPES(FWD_FULL) SHAPES_HALF(FWD_HALF)};
+const Variant BWD[] = {SHAPES(BWD_FULL)};
+constexpr int NFWD = (int)(sizeof(FWD) / sizeof(FWD[0])), NBWD = (int)(sizeof(BWD) / sizeof(BWD[0]));
+constexpr int NMAX = NFWD > NBWD ? NFWD : NBWD;
 
-void launch_config(const Variant &v, bool backward, int clusters, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
+void launch_config(const Variant &v, int clusters, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = v.C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     *cfg = cudaLaunchConfig_t{};
     cfg->gridDim = dim3(clusters * v.C);
     cfg->blockDim = dim3(32 * v.WN);
-    cfg->dynamicSmemBytes = smem_bytes(v, backward);
+    cfg->dynamicSmemBytes = v.smem;
     cfg->stream = st;
     cfg->attrs = attr;
     cfg->numAttrs = 1;
 }
 
-// clusters of a variant the current device holds at once (asked once per kernel and device)
-int resident_clusters(int vi, bool backward) {
+// clusters of a variant that the current device holds at once (asked once per kernel and device)
+// (*alone: with one block per SM)
+int resident_clusters(bool backward, int vi, int *alone) {
     static std::mutex mu;
-    static int known[MAX_DEVICES][NVARIANTS][2];    // 0 = not asked yet, else clusters + 1
+    static short known[MAX_DEVICES][2][NMAX][2];    // 0 = not asked yet, else clusters + 1
     const int dev = current_device();
+    const Variant &v = backward ? BWD[vi] : FWD[vi];
     if (dev < 0) return 0;
     std::lock_guard<std::mutex> lk(mu);
-    int &k = known[dev][vi][backward];
-    if (!k) {
-        const Variant &v = VARIANTS[vi];
-        const Kernel f = backward ? v.bwd : v.fwd;
-        int n = 0;
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[1];
-        launch_config(v, backward, 1, nullptr, &cfg, attr);
-        if (cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(v, backward)) != cudaSuccess ||
-            (v.C > 8 && cudaFuncSetAttribute((const void *)f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-            cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess) {
+    short *k = known[dev][backward][vi];
+    if (!k[0]) {
+        const int spread = 120 * 1024;     // shared memory that keeps a second block off the SM
+        if (cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, spread) != cudaSuccess ||
+            (v.C > 8 && cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
             cudaGetLastError();
-            n = 0;
+        for (int q = 0; q < 2; ++q) {
+            int n = 0;
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute attr[1];
+            launch_config(v, 1, nullptr, &cfg, attr);
+            if (q) cfg.dynamicSmemBytes = spread;
+            if (cudaOccupancyMaxActiveClusters(&n, v.kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+            k[q] = (short)(n + 1);
         }
-        k = n + 1;
     }
-    return k - 1;
+    *alone = k[1] - 1;
+    return k[0] - 1;
 }
 
-// Cycles per step as measured with probes and sweeps: 900 for the chain (first byte of the exchange, gate math), 1 (cluster of
-// 16: 1.2) per 16 bytes a block receives, 8 per MMA of an SM quarter; blocks that share an SM share its tensor cores and network port.
-int pick_variant(const LstmShape &s, bool backward) {
-    int best = -1;
+// Cycles of a step, fitted to sweeps on a B200 at 1.95 GHz (forward / backward, us per step: 256 units on clusters of 16 x 4 warps
+// 0.97 / 0.99, of 8 x 8 warps 1.28 / 1.29; 128 units, 8 x 4: 0.67 / 0.85; 64 units, 4 x 4: 0.60 / 0.75; 16 units, one block: 0.46 /
+// 0.58).  A second warp on an SM quarter adds its own cell math; share = blocks of an SM.
+double step_cycles(const Variant &v, int KP, double share, bool backward) {
+    const int waves = (v.WN + 3) / 4;
+    const double mma = (v.half ? 16.0 : 24.0) * (KP / 16) * waves;
+    const double packets = v.C > 1 ? (v.C > 8 ? 0.7 : 0.4) * KP * (v.half ? 1.0 : 2.0) : 0.0;
+    return (backward ? 850.0 : 620.0) + (v.C > 1 ? 430.0 : 0.0) + 350.0 * (waves - 1) + share * (mma + packets);
+}
+
+struct Plan { int vi, items, clusters; };
+Plan make_plan(const LstmShape &s, bool backward) {
+    Plan best{-1, 0, 0};
     double best_t = 0.0;
-    for (int vi = 0; vi < NVARIANTS; ++vi) {
-        const Variant &v = VARIANTS[vi];
+    const int items = s.D * ((s.P + 7) / 8);
+    for (int vi = 0; vi < (backward ? NBWD : NFWD); ++vi) {
+        const Variant &v = backward ? BWD[vi] : FWD[vi];
         const int KP = v.C * 4 * v.WN;
-        if (KP < s.els) continue;
-        const int res = resident_clusters(vi, backward);
-        if (res < 1) continue;
-        const int items = s.D * ((s.P + 8 * v.NT - 1) / (8 * v.NT));
-        const int passes = (items + res - 1) / res, live = items < res ? items : res;
-        const int share = (live * v.C + sm_count() - 1) / sm_count();
-        const double step = 900.0 + 60.0 * v.NT + share * v.NT * ((v.C > 8 ? 1.2 : 1.0) * KP * 2 + (KP / 16) * 24.0 * ((v.WN + 3) / 4));
-        const double t = passes * step * (1.0 + 1e-4 * live * v.C / sm_count());    // the smaller launch where two are equal
-        if (best < 0 || t < best_t) { best = vi; best_t = t; }
+        if (KP < s.els || (v.half && s.P > 4)) continue;
+        int alone = 0;
+        const int res = resident_clusters(backward, vi, &alone);
+        if (res < 1 || alone < 1) continue;
+        const int live = items < res ? items : res, passes = (items + live - 1) / live;
+        const double share = (double)((live + alone - 1) / alone);
+        // where two come out equal, the one on fewer SMs: another net's kernels may want the rest
+        const double t = passes * step_cycles(v, KP, share, backward) * (1.0 + 0.05 * live * v.C / sm_count());
+        if (best.vi < 0 || t < best_t) { best = Plan{vi, items, live}; best_t = t; }
     }
     return best;
 }
 
 }  // namespace
 
-bool lstm_cluster_supported(const LstmShape &s) { return s.els <= 320 && pick_variant(s, false) >= 0 && pick_variant(s, true) >= 0; }
+bool lstm_cluster_supported(const LstmShape &s) { return s.els <= 320 && make_plan(s, false).vi >= 0 && make_plan(s, true).vi >= 0; }
 
 int lstm_cluster_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
                        cudaStream_t st) {
-    const int vi = pick_variant(s, backward);
-    if (vi < 0) return 1;
-    const Variant &v = VARIANTS[vi];
+    const Plan pl = make_plan(s, backward);
+    if (pl.vi < 0) return 1;
+    const Variant &v = backward ? BWD[pl.vi] : FWD[pl.vi];
     ClusterArgs a;
     a.sh = s; a.bf = b; a.w = w; a.y = y; a.dy = dy; a.status = status;
-    a.n_items = s.D * ((s.P + 8 * v.NT - 1) / (8 * v.NT));
-    const int res = resident_clusters(vi, backward);
-    a.nclusters = a.n_items < res ? a.n_items : res;
+    a.n_items = pl.items; a.nclusters = pl.clusters;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    launch_config(v, backward, a.nclusters, st, &cfg, attr);
-    B2_CUDA(cudaLaunchKernelEx(&cfg, backward ? v.bwd : v.fwd, a));
+    launch_config(v, pl.clusters, st, &cfg, attr);
+    B2_CUDA(cudaLaunchKernelEx(&cfg, v.kern, a));
     count_launch();
     return B2_OK;
 }

@@ -256,6 +256,9 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
             int splits = 0;
             double best = 0.0;
             for (int sp = 1; sp <= 64 && (size_t)sp * 4 * D * per <= ws_floats && (long)sp * 256 <= K; ++sp) {
+                // a split is a whole number of slabs (64 positions of fp16 parts, 32 of tf32 ones); the last one must not be empty
+                const int slab = tcrec_used ? 32 : 64, chunk = ((K + sp - 1) / sp + slab - 1) / slab * slab;
+                if ((long)chunk * (sp - 1) >= K) continue;
                 const int waves = (tiles * sp + sms - 1) / sms;
                 const double t = waves * (0.4 * ((K + sp - 1) / sp) / 64.0 + 3.0) + (double)sp * 4 * D * per * 8.0 / 5.0e6;
                 if (!splits || t < best) { best = t; splits = sp; }
@@ -324,14 +327,11 @@ bool LstmLayerImpl::want_tc_recurrence() const {
     return passes * (1.4 + 0.27 * ps) > 12.0;
 }
 
-// The register-resident cluster kernels serve up to 320 units per direction.  For one or two sequences of the unit counts that
-// have an FFMA geometry those kernels have the shorter step: an MMA always runs 8 sequences.
+// The register-resident cluster kernels serve up to 320 units per direction (what fits the registers of 16 SMs as tensor-core
+// fragments): the shortest step at every number of sequences measured, 1 to 256.  Strict fp32 products (force_ffma) and the other
+// modes stay with the kernels they name.
 bool LstmLayerImpl::want_cluster() const {
-    if (force_ffma || recurrence_mode != 1) return false;
-    const LstmShape s = shape();
-    int JB;
-    if (s.P < 3 && persistent_geometry(s.els, &JB)) return false;
-    return lstm_cluster_supported(s);
+    return !force_ffma && recurrence_mode == 1 && lstm_cluster_supported(shape());
 }
 
 // The persistent tensor-core kernels serve 512 units per direction.  Modes 5 and 6 force them; the default (mode 1)

@@ -554,3 +554,16 @@ def test_cluster_recurrence(els, bi, P, T):
     for key in got:
         if key != "launches":
             assert np.array_equal(np.asarray(got[key]), np.asarray(again[key])), "not deterministic: " + key
+
+
+def test_recurrent_weight_gradient_with_splits_of_whole_slabs():
+    """A contraction length (399 frames x 4 sequences) for which the cheapest number of K splits, rounded to whole slabs, would
+    leave the last split empty."""
+    from b2lstm import workloads
+    layers = L(("input", 6), ("lstm", 128), ("feedforward_identity", 4), ("sse", 4))
+    lens = np.array([400, 400, 390, 100], np.int32)
+    x, tg = workloads.make_fraction(6, 4, 4, lens, 85, 86)
+    w = workloads.make_weights(layers, 87, 0.05)
+    want = run_kind(checker(), layers, 4, lens, x, tg, w)
+    got = run_gpu(layers, 4, lens, x, tg, w, VARIANTS[2])
+    parity.compare_run(layers, got, want, "4 x 400", lstm_pad_zero_lens=lens)
