@@ -197,11 +197,17 @@ int lstm_ptc_prepare(const LstmShape &s, const float *w, const PtcBuffers &pb, c
 int lstm_ptc_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const PtcBuffers &pb, const float *w, float *y,
                    const float *dy, int *status, unsigned *tag_next, cudaStream_t st);
 
-// register-resident tensor-core recurrence on thread-block clusters (lstm_cluster.cu): up to 320 units per direction, any number
+// register-resident tensor-core recurrence on thread-block clusters (lstm_cluster.cu): up to 512 units per direction, any number
 // of sequences.  Returns B2_OK, an error, or 1 when no cluster of the needed size fits on the device.
 bool lstm_cluster_supported(const LstmShape &s);
 int lstm_cluster_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
                        cudaStream_t st);
+
+// FFMA recurrence with one sequence per cluster (lstm_single.cu): up to 512 units per direction, as many (direction, sequence)
+// pairs as clusters fit side by side.  Returns as above.
+bool lstm_single_supported(const LstmShape &s, bool backward);
+int lstm_single_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
+                      cudaStream_t st);
 
 // persistent kernels (lstm_persistent.cu).  Return B2_OK, an error, or 1 when the shape has no
 // persistent kernel (the caller then uses the stepwise kernels).

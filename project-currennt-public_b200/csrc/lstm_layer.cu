@@ -135,9 +135,10 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
         int rc = 1;
         cluster_used = want_cluster();
         if (cluster_used) {
-            rc = lstm_cluster_sweep(false, s, bufs, w, y, nullptr, status_dev, st);
-            fwd_path = 7;
-            if (rc == 1) cluster_used = false;
+            const bool single = lstm_single_supported(s, false);
+            rc = single ? lstm_single_sweep(false, s, bufs, w, y, nullptr, status_dev, st)
+                        : lstm_cluster_sweep(false, s, bufs, w, y, nullptr, status_dev, st);
+            fwd_path = single ? 1 : 7;
         }
         ptc_used = !cluster_used && want_ptc();
         if (ptc_used) {
@@ -177,8 +178,10 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
         Phase ph(*this, "lstm_bwd_recurrence");
         int rc = 1;
         if (cluster_used) {
-            rc = lstm_cluster_sweep(true, s, bufs, w, nullptr, dy, status_dev, st);
-            bwd_path = 7;
+            const bool single = lstm_single_supported(s, true);
+            rc = single ? lstm_single_sweep(true, s, bufs, w, nullptr, dy, status_dev, st)
+                        : lstm_cluster_sweep(true, s, bufs, w, nullptr, dy, status_dev, st);
+            bwd_path = single ? 1 : 7;
         } else if (ptc_used && recurrence_mode != 6) {
             rc = lstm_ptc_sweep(true, s, bufs, ptc, w, nullptr, dy, status_dev, &tag_next, st);
             bwd_path = 5;
@@ -327,17 +330,19 @@ bool LstmLayerImpl::want_tc_recurrence() const {
     return passes * (1.4 + 0.27 * ps) > 12.0;
 }
 
-// The register-resident cluster kernels serve up to 320 units per direction (what fits the registers of 16 SMs as tensor-core
-// fragments): the shortest step at every number of sequences measured, 1 to 256.  Strict fp32 products (force_ffma) and the other
+// The register-resident cluster kernels serve up to 512 units per direction (what the registers and tensor memory of 16 SMs hold):
+// the shortest step wherever the kernels below have none, and for 512 units up to 192 (direction, sequence) pairs, where the chunks of
+// lstm_ptc.cu start to pay (B200, us per step forward / backward, bidirectional: 32 sequences 3.3 / 4.0 here, 4.1 / 4.9 there; 64: 4.7 /
+// 5.9 and 7.2 / 5.5; 128: 9.3 / 10.1 and 9.5 / 10.0; 256: 16.2 / 19.8 and 10.6 / 13.6).  Strict fp32 products (force_ffma) and the other
 // modes stay with the kernels they name.
 bool LstmLayerImpl::want_cluster() const {
-    return !force_ffma && recurrence_mode == 1 && lstm_cluster_supported(shape());
+    const LstmShape s = shape();
+    if (force_ffma || recurrence_mode != 1 || !lstm_cluster_supported(s)) return false;
+    return s.D * s.P <= 192 || !lstm_ptc_supported(s);
 }
 
 // The persistent tensor-core kernels serve 512 units per direction.  Modes 5 and 6 force them; the default (mode 1)
-// takes them from 16 parallel sequences on: measured on B200 with 32 sequences a step costs 4.5 us against 6.1 us of
-// the register-resident FFMA kernels, and the gap widens with the batch (the FFMA kernels' step grows by 0.27 us per
-// sequence of a work item).  Below that the FFMA kernels have the shorter step (1.65 us for one sequence).
+// takes them for fractions too large for the cluster kernels (above).
 bool LstmLayerImpl::want_ptc() const {
     const LstmShape s = shape();
     if (force_ffma || !lstm_ptc_supported(s)) return false;
