@@ -84,13 +84,12 @@ struct TcScratch {
     float *take(size_t floats);
     void release();
 };
-size_t split_floats(int outer, int inner, bool f16 = true);
+size_t split_floats(int outer, int inner);
 int split_tf32(const float *src, long s_outer, int outer, int inner, float *hi, float *lo, long ldp, cudaStream_t st);
-// bound > 0: the caller's promise that no |entry| exceeds it (saves the pass that finds the largest entry)
-int split_f16(const float *src, long s_outer, int outer, int inner, void *hi, void *lo, long ldp, unsigned *maxbits,
-              cudaStream_t st, float bound = 0.0f);
-int split_operand(TcScratch &sc, const float *src, long s_outer, int outer, int inner, bool kmajor, SplitOperand *out,
-                  cudaStream_t st, bool f16 = true, float bound = 0.0f);
+// One operand to be split into fp16 parts: `outer` rows of `inner` contiguous entries, rows s_outer floats apart.  bound > 0: the
+// caller's promise that no |entry| exceeds it (saves the pass that finds the largest entry).  *out receives the parts.
+struct SplitJob { const float *src; long s_outer; int outer, inner; bool kmajor; float bound; SplitOperand *out; };
+int split_operands(TcScratch &sc, const SplitJob *jobs, int n, cudaStream_t st);
 bool gemm_tc_supported(const SplitOperand &A, const SplitOperand &B, int m, int n, int k);
 int gemm_tc(float *C, long ldc, const SplitOperand &A, const SplitOperand &B, int m, int n, int k, bool accumulate,
             float *ws, size_t ws_floats, int *status, cudaStream_t st);
@@ -113,7 +112,7 @@ bool gemm_wants_tc(long sam, long sak, long sbk, long sbn, int m, int n, int k);
 // picks the tensor-core kernel when the shape qualifies (and sc/status are given), else FFMA
 int gemm_auto(float *C, long ldc, const float *A, long sam, long sak, const float *B, long sbk, long sbn, int m, int n,
               int k, bool accumulate, bool force_ffma, TcScratch *sc, float *ws, size_t ws_floats, int *status,
-              cudaStream_t st);
+              cudaStream_t st, float b_bound = 0.0f);   // b_bound: as SplitJob::bound, for B
 
 // ---- feed-forward / loss / optimizer elementwise kernels (elementwise.cu) -------------------------
 // y[f*ls + u] = act(y + bias*b[u]) over n = frames*ls elements

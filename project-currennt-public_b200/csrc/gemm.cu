@@ -28,38 +28,10 @@ float *TcScratch::take(size_t floats) {
     return p;
 }
 
-// split a strided matrix view whose contiguous index has `inner` entries and whose other index has
-// `outer` entries `s_outer` floats apart; returns the dense operand description
-int split_operand(TcScratch &sc, const float *src, long s_outer, int outer, int inner, bool kmajor, SplitOperand *out,
-                  cudaStream_t st, bool f16, float bound) {
-    if (!f16) {
-        const long ldp = (inner + 3) & ~3L;
-        float *hi = sc.take((size_t)outer * ldp), *lo = sc.take((size_t)outer * ldp);
-        if (!hi || !lo) { set_error("split_operand: operand arena exhausted"); return B2_ERR_BAD_SHAPE; }
-        B2_TRY(split_tf32(src, s_outer, outer, inner, hi, lo, ldp, st));
-        *out = SplitOperand{};
-        out->hi = hi; out->lo = lo; out->ld = ldp; out->kmajor = kmajor;
-        return B2_OK;
-    }
-    // fp16 parts: rows padded to 8 halves (16 bytes, what a tensor map wants of a row pitch)
-    const long ldp = (inner + 7) & ~7L;
-    const size_t part = ((size_t)outer * ldp + 1) / 2;   // floats that hold one part
-    float *hi = sc.take(part), *lo = sc.take(part), *mx = sc.take(1);
-    if (!hi || !lo || !mx) { set_error("split_operand: operand arena exhausted"); return B2_ERR_BAD_SHAPE; }
-    B2_TRY(split_f16(src, s_outer, outer, inner, hi, lo, ldp, (unsigned *)mx, st, bound));
-    out->hi = hi; out->lo = lo; out->ld = ldp; out->kmajor = kmajor;
-    out->f16 = true; out->maxbits = (const unsigned *)mx;
-    return B2_OK;
-}
-
-size_t split_floats(int outer, int inner, bool f16) {
-    if (!f16) {
-        const size_t ldp = (size_t)((inner + 3) & ~3);
-        return 2 * (((size_t)outer * ldp + 63) & ~(size_t)63);
-    }
+size_t split_floats(int outer, int inner) {
     const size_t ldp = (size_t)((inner + 7) & ~7);
     const size_t part = ((size_t)outer * ldp + 1) / 2;
-    return 2 * ((part + 63) & ~(size_t)63) + 64;
+    return 2 * ((part + 63) & ~(size_t)63) + 704;      // both parts, scale word and partial maxima
 }
 
 bool gemm_wants_tc(long sam, long sak, long sbk, long sbn, int m, int n, int k) {
@@ -70,7 +42,7 @@ bool gemm_wants_tc(long sam, long sak, long sbk, long sbn, int m, int n, int k) 
 }
 
 int gemm_auto(float *C, long ldc, const float *A, long sam, long sak, const float *B, long sbk, long sbn, int m, int n, int k,
-              bool accumulate, bool force_ffma, TcScratch *sc, float *ws, size_t ws_floats, int *status, cudaStream_t st) {
+              bool accumulate, bool force_ffma, TcScratch *sc, float *ws, size_t ws_floats, int *status, cudaStream_t st, float b_bound) {
     if (force_ffma || !sc || !status || !gemm_wants_tc(sam, sak, sbk, sbn, m, n, k))
         return gemm_ffma(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, accumulate, ws, ws_floats, st);
     const bool a_k = (sak == 1), b_k = (sbk == 1);
@@ -79,8 +51,8 @@ int gemm_auto(float *C, long ldc, const float *A, long sam, long sak, const floa
     B2_TRY(sc->reserve(split_floats(a_outer, a_inner) + split_floats(b_outer, b_inner)));
     sc->used = 0;
     SplitOperand sa, sb;
-    B2_TRY(split_operand(*sc, A, a_k ? sam : sak, a_outer, a_inner, a_k, &sa, st));
-    B2_TRY(split_operand(*sc, B, b_k ? sbn : sbk, b_outer, b_inner, b_k, &sb, st));
+    const SplitJob jobs[2] = {{A, a_k ? sam : sak, a_outer, a_inner, a_k, 0.0f, &sa}, {B, b_k ? sbn : sbk, b_outer, b_inner, b_k, b_bound, &sb}};
+    B2_TRY(split_operands(*sc, jobs, 2, st));
     return gemm_tc(C, ldc, sa, sb, m, n, k, accumulate, ws, ws_floats, status, st);
 }
 

@@ -110,6 +110,63 @@ __global__ void __launch_bounds__(NT) gemm_ffma_kernel(float *__restrict__ C, lo
     }
 }
 
+// Small products (a handful of 128 x 128 tiles would leave the chip idle and each tile's K loop serial): 32 x 32 tiles, 128 threads
+// with 2 x 4 accumulators, K slabs of 32.  Same order of summation per output as above.
+constexpr int SM_T = 32, SM_K = 32, SM_NT = 128;
+template <bool A_ROW_FAST, bool B_COL_FAST>
+__global__ void __launch_bounds__(SM_NT) gemm_ffma_small_kernel(float *__restrict__ C, long ldc, const float *__restrict__ A, long sam,
+                                                                long sak, const float *__restrict__ B, long sbk, long sbn, int M, int N,
+                                                                int K, int kchunk, int accumulate, float *__restrict__ ws) {
+    __shared__ __align__(16) float As[SM_K][SM_T + 4], Bs[SM_K][SM_T + 4];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;     // rows 2 tx, 2 tx + 1; columns 4 ty .. + 3
+    const int m0 = blockIdx.x * SM_T, n0 = blockIdx.y * SM_T, kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
+    float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    float ra[8], rb[8];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int e = tid + i * SM_NT;
+            const int ar = A_ROW_FAST ? e % SM_T : e / SM_K, ak = A_ROW_FAST ? e / SM_T : e % SM_K;
+            const int br = B_COL_FAST ? e % SM_T : e / SM_K, bk = B_COL_FAST ? e / SM_T : e % SM_K;
+            ra[i] = (m0 + ar < M && k0 + ak < kend) ? __ldg(A + (long)(m0 + ar) * sam + (long)(k0 + ak) * sak) : 0.0f;
+            rb[i] = (n0 + br < N && k0 + bk < kend) ? __ldg(B + (long)(n0 + br) * sbn + (long)(k0 + bk) * sbk) : 0.0f;
+        }
+    };
+    load(kbeg);
+    for (int k0 = kbeg; k0 < kend; k0 += SM_K) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int e = tid + i * SM_NT;
+            As[A_ROW_FAST ? e / SM_T : e % SM_K][A_ROW_FAST ? e % SM_T : e / SM_K] = ra[i];
+            Bs[B_COL_FAST ? e / SM_T : e % SM_K][B_COL_FAST ? e % SM_T : e / SM_K] = rb[i];
+        }
+        __syncthreads();
+        if (k0 + SM_K < kend) load(k0 + SM_K);
+#pragma unroll 8
+        for (int kk = 0; kk < SM_K; ++kk) {
+            const float2 a = *(const float2 *)&As[kk][2 * tx];
+            const float4 b = *(const float4 *)&Bs[kk][4 * ty];
+            acc[0][0] = fmaf(a.x, b.x, acc[0][0]); acc[0][1] = fmaf(a.x, b.y, acc[0][1]);
+            acc[0][2] = fmaf(a.x, b.z, acc[0][2]); acc[0][3] = fmaf(a.x, b.w, acc[0][3]);
+            acc[1][0] = fmaf(a.y, b.x, acc[1][0]); acc[1][1] = fmaf(a.y, b.y, acc[1][1]);
+            acc[1][2] = fmaf(a.y, b.z, acc[1][2]); acc[1][3] = fmaf(a.y, b.w, acc[1][3]);
+        }
+        __syncthreads();
+    }
+    const bool split = gridDim.z > 1;
+    float *dst = split ? ws + (size_t)blockIdx.z * (size_t)M * N : C;
+    const long ld = split ? (long)M : ldc;
+#pragma unroll
+    for (int jn = 0; jn < 4; ++jn)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int m = m0 + 2 * tx + i, n = n0 + 4 * ty + jn;
+            if (m >= M || n >= N) continue;
+            float *p = dst + (long)n * ld + m;
+            *p = !split && accumulate ? acc[i][jn] + *p : acc[i][jn];
+        }
+}
+
 __global__ void splitk_reduce_kernel(float *__restrict__ C, long ldc, const float *__restrict__ ws, int M, int N,
                                      int splits, int accumulate) {
     size_t total = (size_t)M * N;
@@ -135,26 +192,35 @@ int gemm_ffma(float *C, long ldc, const float *A, long sam, long sak, const floa
         return B2_OK;
     }
     dim3 grid((m + BM - 1) / BM, (n + BN - 1) / BN, 1);
-    // split K when the output tiles alone cannot fill the GPU and K is long
-    int tiles = grid.x * grid.y;
-    int splits = 1;
     const int sms = sm_count();
-    if (ws && tiles < sms && k >= 2048) {
+    // Fewer 128 x 128 tiles than a quarter of the SMs: the small tiles (128 x 800 x 32, the error of a 32-unit output layer over 800
+    // frames: 7 tiles of 128 x 128, 26 us; 100 of 32 x 32, 4 us).  K is split when the tiles alone cannot fill the GPU: from two chunks
+    // of 512 (small tiles: 64) positions on.
+    const bool small = (int)(grid.x * grid.y) * 4 < sms;
+    if (small) grid = dim3((m + SM_T - 1) / SM_T, (n + SM_T - 1) / SM_T, 1);
+    const int tiles = grid.x * grid.y, least = small ? 64 : 512;
+    int splits = 1;
+    if (ws && tiles < sms && k >= (small ? 2 : 4) * least) {
         splits = (2 * sms + tiles - 1) / tiles;
-        int maxs = k / 512;
+        int maxs = k / least;
         if (splits > maxs) splits = maxs;
         size_t per = (size_t)m * n;
         if (per && (size_t)splits * per > ws_floats) splits = (int)(ws_floats / per);
         if (splits < 1) splits = 1;
     }
+    const int slab = small ? SM_K : BK;
     int kchunk = (k + splits - 1) / splits;
-    kchunk = (kchunk + BK - 1) / BK * BK;
+    kchunk = (kchunk + slab - 1) / slab * slab;
     splits = (k + kchunk - 1) / kchunk;
     grid.z = splits;
     const bool a_row = (sam == 1), b_col = (sbn == 1);
-#define LAUNCH(AR, BC)                                                                                     \
-    gemm_ffma_kernel<AR, BC><<<grid, NT, 0, st>>>(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, kchunk, \
-                                                  accumulate ? 1 : 0, ws)
+#define LAUNCH(AR, BC)                                                                                                            \
+    do {                                                                                                                          \
+        if (small)                                                                                                                \
+            gemm_ffma_small_kernel<AR, BC><<<grid, SM_NT, 0, st>>>(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, kchunk, accumulate ? 1 : 0, ws); \
+        else                                                                                                                      \
+            gemm_ffma_kernel<AR, BC><<<grid, NT, 0, st>>>(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, kchunk, accumulate ? 1 : 0, ws);          \
+    } while (0)
     if (a_row && b_col) LAUNCH(true, true);
     else if (a_row) LAUNCH(true, false);
     else if (b_col) LAUNCH(false, true);

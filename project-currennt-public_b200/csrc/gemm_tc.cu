@@ -518,40 +518,71 @@ __global__ void __launch_bounds__(256) split_tf32_vec4_kernel(const float *__res
     }
 }
 
-// ---- fp16 parts.  The largest finite |x| of the operand first (bit pattern, atomicMax), then the split with the scale that follows from it.
-__global__ void __launch_bounds__(256) absmax_kernel(const float *__restrict__ src, long s_outer, int outer, int inner, int vec4,
-                                                     unsigned *maxbits) {
-    unsigned m = 0u;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    if (vec4) {
-        const int inner4 = inner / 4;
-        const size_t total = (size_t)outer * inner4;
-        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-            const float4 x = __ldg((const float4 *)(src + (i / inner4) * s_outer) + (i % inner4));
-            const unsigned b0 = __float_as_uint(fabsf(x.x)), b1 = __float_as_uint(fabsf(x.y));
-            const unsigned b2 = __float_as_uint(fabsf(x.z)), b3 = __float_as_uint(fabsf(x.w));
-            if (b0 < 0x7f800000u) m = max(m, b0);   // NaN / Inf do not set the scale
-            if (b1 < 0x7f800000u) m = max(m, b1);
-            if (b2 < 0x7f800000u) m = max(m, b2);
-            if (b3 < 0x7f800000u) m = max(m, b3);
-        }
-    } else {
-        const size_t total = (size_t)outer * inner;
-        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-            const unsigned b = __float_as_uint(fabsf(src[(i / inner) * s_outer + (i % inner)]));
-            if (b < 0x7f800000u) m = max(m, b);
-        }
-    }
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+// ---- fp16 parts: all operands of a product (or of a layer's products) in at most two launches.  The first finds the largest finite
+// |x| of the operands that come without a bound, one partial result per block; the second reduces those (every block for itself: a
+// few hundred words from L2), derives the scale and splits.  Bandwidth decides the large operands (read 4, read 4 and write 4 bytes
+// an entry), launches the small ones: a memset and two kernels per operand made 8 launches of a layer's backward pass.
+constexpr int MAX_SPLIT_JOBS = 4, MAX_SPLIT_BLOCKS = 592;
+struct SplitWork {
+    const float *src;
+    long s_outer;
+    int outer, inner;
+    unsigned short *hi, *lo;   // [outer][ldp] halves, zero padded to ldp
+    long ldp;
+    unsigned bound;            // bit pattern of the caller's bound; 0: none
+    unsigned *maxbits;         // receives the bit pattern the scale follows from
+    unsigned *partial;         // the blocks' maxima
+    int vec, parts;            // 16-byte accesses possible; blocks (= partial results)
+};
+struct SplitBatch { SplitWork w[MAX_SPLIT_JOBS]; int first[MAX_SPLIT_JOBS + 1]; };   // first block of each job
+
+__device__ __forceinline__ unsigned block_max256(unsigned m) {
     __shared__ unsigned wm[8];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) m = max(m, wm[w]);
-        if (m) atomicMax(maxbits, m);
-    }
+    m = wm[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = max(m, wm[w]);
+    return m;
 }
-__global__ void set_word_kernel(unsigned *dst, unsigned v) { *dst = v; }
+__device__ __forceinline__ unsigned finite_bits(float x) {
+    const unsigned b = __float_as_uint(fabsf(x));
+    return b < 0x7f800000u ? b : 0u;     // NaN / Inf do not set the scale
+}
+// the job of this block, its index among the job's blocks
+__device__ __forceinline__ const SplitWork &split_job(const SplitBatch &sb, int &block) {
+    int j = 0;
+    while (j + 1 < MAX_SPLIT_JOBS && (int)blockIdx.x >= sb.first[j + 1]) ++j;
+    block = (int)blockIdx.x - sb.first[j];
+    return sb.w[j];
+}
+__global__ void __launch_bounds__(256) absmax_batch_kernel(const __grid_constant__ SplitBatch sb) {
+    int block;
+    const SplitWork &w = split_job(sb, block);
+    unsigned m = 0u;
+    const size_t stride = (size_t)w.parts * 256, i0 = (size_t)block * 256 + threadIdx.x;
+    if (w.vec) {
+        const unsigned in4 = (unsigned)w.inner / 4;
+        const size_t total = (size_t)w.outer * in4;
+        const bool dense = w.s_outer == w.inner;
+        for (size_t i = i0; i < total; i += stride) {
+            const float4 x = __ldg(dense ? (const float4 *)w.src + i : (const float4 *)(w.src + (i / in4) * w.s_outer) + i % in4);
+            m = max(m, max(max(finite_bits(x.x), finite_bits(x.y)), max(finite_bits(x.z), finite_bits(x.w))));
+        }
+    } else if (w.s_outer == w.inner) {
+        const size_t total = (size_t)w.outer * w.inner;
+#pragma unroll 4
+        for (size_t i = i0; i < total; i += stride) m = max(m, finite_bits(__ldg(w.src + i)));
+    } else {
+        // a warp per row
+        for (int r = block * 8 + (int)(threadIdx.x >> 5); r < w.outer; r += w.parts * 8)
+            for (int c = threadIdx.x & 31; c < w.inner; c += 32) m = max(m, finite_bits(__ldg(w.src + (size_t)r * w.s_outer + c)));
+    }
+    m = block_max256(m);
+    if (threadIdx.x == 0) w.partial[block] = m;
+}
 inline unsigned float_bits(float f) { unsigned u; memcpy(&u, &f, sizeof u); return u; }
 // x*S = hi + lo * 2^-11; both parts as fp16 bit patterns
 __device__ __forceinline__ void split_f16_one(float x, float S, unsigned short &h, unsigned short &l) {
@@ -561,35 +592,37 @@ __device__ __forceinline__ void split_f16_one(float x, float S, unsigned short &
     h = __half_as_ushort(hh);
     l = __half_as_ushort(ll);
 }
-// dense destination [outer][ldp] halves, zero padded to ldp
-__global__ void split_f16_kernel(const float *__restrict__ src, long s_outer, int outer, int inner, unsigned short *__restrict__ hi,
-                                 unsigned short *__restrict__ lo, long ldp, const unsigned *__restrict__ maxbits) {
-    const float S = ldexpf(1.0f, f16_scale_exp(*maxbits));
-    const size_t total = (size_t)outer * ldp;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t o = i / ldp;
-        const int c = (int)(i % ldp);
-        const float x = c < inner ? src[o * s_outer + c] : 0.0f;
-        split_f16_one(x, S, hi[i], lo[i]);
+// a thread writes 8 consecutive entries of both parts (16 bytes each)
+__global__ void __launch_bounds__(256) split_f16_batch_kernel(const __grid_constant__ SplitBatch sb) {
+    int block;
+    const SplitWork &w = split_job(sb, block);
+    unsigned m = w.bound;
+    if (!m) {
+        for (int i = threadIdx.x; i < w.parts; i += 256) m = max(m, __ldg(w.partial + i));
+        m = block_max256(m);
     }
-}
-// rows that are whole groups of 8 (inner == ldp, a multiple of 8; bases and the source stride 16-byte aligned)
-__global__ void __launch_bounds__(256) split_f16_vec8_kernel(const float *__restrict__ src, long s_outer, int outer, int inner8,
-                                                             uint4 *__restrict__ hi, uint4 *__restrict__ lo,
-                                                             const unsigned *__restrict__ maxbits) {
-    const float S = ldexpf(1.0f, f16_scale_exp(*maxbits));
-    const size_t total = (size_t)outer * inner8;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 *p = (const float4 *)(src + (i / inner8) * s_outer) + 2 * (i % inner8);
-        const float4 x0 = __ldg(p), x1 = __ldg(p + 1);
-        const float in[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    if (block == 0 && threadIdx.x == 0) *w.maxbits = m;
+    const float S = ldexpf(1.0f, f16_scale_exp(m));
+    const unsigned ld8 = (unsigned)(w.ldp / 8);
+    const size_t total = (size_t)w.outer * ld8;
+    for (size_t i = (size_t)block * 256 + threadIdx.x; i < total; i += (size_t)w.parts * 256) {
+        const unsigned r = total <= 0xffffffffu ? (unsigned)i / ld8 : (unsigned)(i / ld8), c = (unsigned)(i - (size_t)r * ld8) * 8u;
+        const float *p = w.src + (size_t)r * w.s_outer + c;
+        float in[8];
+        if (w.vec) {
+            const float4 x0 = __ldg((const float4 *)p), x1 = c + 4 < (unsigned)w.inner ? __ldg((const float4 *)p + 1) : make_float4(0, 0, 0, 0);
+            in[0] = x0.x; in[1] = x0.y; in[2] = x0.z; in[3] = x0.w; in[4] = x1.x; in[5] = x1.y; in[6] = x1.z; in[7] = x1.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) in[e] = c + e < (unsigned)w.inner ? __ldg(p + e) : 0.0f;
+        }
         unsigned short h[8], l[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) split_f16_one(in[e], S, h[e], l[e]);
-        hi[i] = make_uint4(h[0] | ((unsigned)h[1] << 16), h[2] | ((unsigned)h[3] << 16), h[4] | ((unsigned)h[5] << 16),
-                           h[6] | ((unsigned)h[7] << 16));
-        lo[i] = make_uint4(l[0] | ((unsigned)l[1] << 16), l[2] | ((unsigned)l[3] << 16), l[4] | ((unsigned)l[5] << 16),
-                           l[6] | ((unsigned)l[7] << 16));
+        ((uint4 *)w.hi)[i] = make_uint4(h[0] | ((unsigned)h[1] << 16), h[2] | ((unsigned)h[3] << 16), h[4] | ((unsigned)h[5] << 16),
+                                        h[6] | ((unsigned)h[7] << 16));
+        ((uint4 *)w.lo)[i] = make_uint4(l[0] | ((unsigned)l[1] << 16), l[2] | ((unsigned)l[3] << 16), l[4] | ((unsigned)l[5] << 16),
+                                        l[6] | ((unsigned)l[7] << 16));
     }
 }
 
@@ -683,39 +716,39 @@ int split_tf32(const float *src, long s_outer, int outer, int inner, float *hi, 
     return B2_OK;
 }
 
-// fp16 parts of a strided matrix view: hi / lo hold [outer][ldp] halves (ldp a multiple of 8), maxbits one word that
-// receives the bit pattern of the largest finite |x| (the scale follows from it, on the device)
-int split_f16(const float *src, long s_outer, int outer, int inner, void *hi, void *lo, long ldp, unsigned *maxbits,
-              cudaStream_t st, float bound) {
-    const size_t total = (size_t)outer * ldp;
-    if (!total) return B2_OK;
-    const bool v4 = (inner % 4) == 0 && (s_outer % 4) == 0 && ((uintptr_t)src % 16) == 0;
-    if (bound > 0.0f) {
-        // the caller knows that no entry exceeds `bound`: the scale follows from it, the pass over the operand is saved
-        set_word_kernel<<<1, 1, 0, st>>>(maxbits, float_bits(bound));
-        count_launch();
-        B2_CUDA(cudaGetLastError());
-    } else {
-        B2_CUDA(cudaMemsetAsync(maxbits, 0, sizeof(unsigned), st));
-        const size_t work = v4 ? (size_t)outer * (inner / 4) : (size_t)outer * inner;
-        size_t blocks = (work + 1023) / 1024;
-        if (blocks > (size_t)sm_count() * 8) blocks = (size_t)sm_count() * 8;
-        if (blocks < 1) blocks = 1;
-        absmax_kernel<<<(int)blocks, 256, 0, st>>>(src, s_outer, outer, inner, v4 ? 1 : 0, maxbits);
-        count_launch();
-        B2_CUDA(cudaGetLastError());
+// fp16 parts of up to MAX_SPLIT_JOBS strided matrix views, out of the arena; the scale follows from a device word, no host round trip
+int split_operands(TcScratch &sc, const SplitJob *jobs, int n, cudaStream_t st) {
+    SplitBatch sb{}, mx{};
+    int nmx = 0;
+    if (n < 1 || n > MAX_SPLIT_JOBS) { set_error("split_operands: 1..%d operands", MAX_SPLIT_JOBS); return B2_ERR_BAD_ARG; }
+    for (int j = 0; j < n; ++j) {
+        const SplitJob &q = jobs[j];
+        SplitWork &w = sb.w[j];
+        // rows padded to 8 halves (16 bytes, what a tensor map wants of a row pitch)
+        w.ldp = (q.inner + 7) & ~7L;
+        const size_t part = ((size_t)q.outer * w.ldp + 1) / 2;   // floats that hold one part
+        float *hi = sc.take(part), *lo = sc.take(part), *mb = sc.take(64 + MAX_SPLIT_BLOCKS);
+        if (!hi || !lo || !mb) { set_error("split_operands: operand arena exhausted"); return B2_ERR_BAD_SHAPE; }
+        w.src = q.src; w.s_outer = q.s_outer; w.outer = q.outer; w.inner = q.inner;
+        w.hi = (unsigned short *)hi; w.lo = (unsigned short *)lo;
+        w.bound = q.bound > 0.0f ? float_bits(q.bound) : 0u;
+        w.maxbits = (unsigned *)mb; w.partial = (unsigned *)mb + 64;
+        w.vec = (q.inner % 4) == 0 && (q.s_outer % 4) == 0 && ((uintptr_t)q.src % 16) == 0;
+        const size_t groups = (size_t)q.outer * (w.ldp / 8), want = (groups + 511) / 512;
+        w.parts = (int)(want < 1 ? 1 : (want > MAX_SPLIT_BLOCKS ? MAX_SPLIT_BLOCKS : want));
+        sb.first[j + 1] = sb.first[j] + w.parts;
+        if (!w.bound) { mx.w[nmx] = w; mx.first[nmx + 1] = mx.first[nmx] + w.parts; ++nmx; }
+        SplitOperand &o = *q.out;
+        o = SplitOperand{};
+        o.hi = hi; o.lo = lo; o.ld = w.ldp; o.kmajor = q.kmajor; o.f16 = true; o.maxbits = w.maxbits;
     }
-    if (v4 && (inner % 8) == 0 && ldp == inner && ((uintptr_t)hi % 16) == 0 && ((uintptr_t)lo % 16) == 0) {
-        const size_t groups = total / 8;
-        size_t blocks = (groups + 255) / 256;
-        if (blocks > (size_t)sm_count() * 16) blocks = (size_t)sm_count() * 16;
-        split_f16_vec8_kernel<<<(int)blocks, 256, 0, st>>>(src, s_outer, outer, inner / 8, (uint4 *)hi, (uint4 *)lo, maxbits);
-    } else {
-        size_t blocks = (total + 255) / 256;
-        if (blocks > (size_t)sm_count() * 16) blocks = (size_t)sm_count() * 16;
-        split_f16_kernel<<<(int)blocks, 256, 0, st>>>(src, s_outer, outer, inner, (unsigned short *)hi, (unsigned short *)lo, ldp,
-                                                      maxbits);
+    for (int j = n; j < MAX_SPLIT_JOBS; ++j) sb.first[j + 1] = 1 << 30;
+    for (int j = nmx; j < MAX_SPLIT_JOBS; ++j) mx.first[j + 1] = 1 << 30;
+    if (nmx) {
+        absmax_batch_kernel<<<mx.first[nmx], 256, 0, st>>>(mx);
+        count_launch();
     }
+    split_f16_batch_kernel<<<sb.first[n], 256, 0, st>>>(sb);
     count_launch();
     B2_CUDA(cudaGetLastError());
     return B2_OK;

@@ -128,7 +128,8 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
     // LstmLayer.cu:1756-1775): acts(4ls x N) = W_in^T X, W_in viewed as ONE pls x 4ls matrix
     {
         Phase ph(*this, "lstm_proj_gemm");
-        B2_TRY(gemm(bufs.acts, 4 * ls, w, pls, 1, x, 1, pls, 4 * ls, N, pls, false, st));
+        B2_TRY(gemm_auto(bufs.acts, 4 * ls, w, pls, 1, x, 1, pls, 4 * ls, N, pls, false, force_ffma, scratch, ws, ws_floats, status_dev, st,
+                         x_bound));
     }
     {
         Phase ph(*this, "lstm_fwd_recurrence");
@@ -202,22 +203,13 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
         // every operand of the four contractions is split into hi/lo parts ONCE and reused:
         // deltas feed dX, dW_in and dW_rec; the layouts [frame][unit] serve both as K-major and
         // as MN-major operands, only the role of the contiguous index changes
-        Phase ph(*this, "lstm_split_tf32");
-        const bool f16 = !tcrec_used;   // the per-timestep tensor-core recurrence leaves tf32 parts: its partners follow
-        B2_TRY(scratch->reserve(split_floats(N, 4 * ls, f16) + split_floats(N, pls, f16) + split_floats(N, ls, f16) +
-                                split_floats(4 * ls, pls, f16)));
+        Phase ph(*this, "lstm_split");
+        B2_TRY(scratch->reserve(split_floats(N, 4 * ls) + split_floats(N, pls) + split_floats(N, ls) + split_floats(4 * ls, pls)));
         scratch->used = 0;
-        if (tcrec_used) {
-            // the tensor-core recurrence has already written the hi/lo parts of the deltas and of y
-            sD.hi = tcrec.d_hi; sD.lo = tcrec.d_lo; sD.ld = 4 * ls; sD.kmajor = true;
-            sY.hi = tcrec.y_hi; sY.lo = tcrec.y_lo; sY.ld = ls; sY.kmajor = false;
-        } else {
-            // the gate deltas are clipped to [-1, 1] (helpers/limitedError.cuh of the reference), |h| = |tanh(c) * og| < 1
-            B2_TRY(split_operand(*scratch, bufs.deltas, 4 * ls, N, 4 * ls, true, &sD, st, true, 1.0f));
-            B2_TRY(split_operand(*scratch, y, ls, N, ls, false, &sY, st, true, 1.0f));
-        }
-        B2_TRY(split_operand(*scratch, x, pls, N, pls, false, &sX, st, f16));
-        B2_TRY(split_operand(*scratch, w, pls, 4 * ls, pls, false, &sW, st, f16));
+        // the gate deltas are clipped to [-1, 1] (helpers/limitedError.cuh of the reference), |h| = |tanh(c) * og| < 1
+        const SplitJob jobs[4] = {{bufs.deltas, 4L * ls, N, 4 * ls, true, 1.0f, &sD}, {y, ls, N, ls, false, 1.0f, &sY},
+                                  {x, pls, N, pls, false, x_bound, &sX}, {w, pls, 4 * ls, pls, false, 0.0f, &sW}};
+        B2_TRY(split_operands(*scratch, jobs, dx ? 4 : 3, st));
     }
     // error to the preceding layer (reference: 4*D Sgemm, LstmLayer.cu:2298-2334): dX = W_in * deltas
     if (dx) {
@@ -246,9 +238,9 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
     //   dW_rec[g][d](k, j) = sum_f h_d[k; f -/+ P] * delta_g,d[j; f], skipping the first (last) timestep
     {
         Phase ph(*this, "lstm_dw_rec_gemm");
-        // the boxes of both operands start at column g*ls + d*els: a TMA copy must start on a 16-byte boundary (8 halves,
-        // 4 floats), other unit counts take the FFMA kernel
-        const bool tc_rec = tc && (els % (tcrec_used ? 4 : 8)) == 0 && gemm_wants_tc(1, ls, 4 * ls, 1, els, els, K);
+        // the boxes of both operands start at column g*ls + d*els: a TMA copy must start on a 16-byte boundary (8 halves),
+        // other unit counts take the FFMA kernel
+        const bool tc_rec = tc && (els % 8) == 0 && gemm_wants_tc(1, ls, 4 * ls, 1, els, els, K);
         bool done = false;
         if (tc_rec && 4 * D <= 8) {
             // all 4*D products in ONE batched launch: batch = (direction, gate); K is split so that the
@@ -259,8 +251,8 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
             int splits = 0;
             double best = 0.0;
             for (int sp = 1; sp <= 64 && (size_t)sp * 4 * D * per <= ws_floats && (long)sp * 256 <= K; ++sp) {
-                // a split is a whole number of slabs (64 positions of fp16 parts, 32 of tf32 ones); the last one must not be empty
-                const int slab = tcrec_used ? 32 : 64, chunk = ((K + sp - 1) / sp + slab - 1) / slab * slab;
+                // a split is a whole number of slabs of 64 positions; the last one must not be empty
+                const int chunk = ((K + sp - 1) / sp + 63) / 64 * 64;
                 if ((long)chunk * (sp - 1) >= K) continue;
                 const int waves = (tiles * sp + sms - 1) / sms;
                 const double t = waves * (0.4 * ((K + sp - 1) / sp) / 64.0 + 3.0) + (double)sp * 4 * D * per * 8.0 / 5.0e6;

@@ -11,6 +11,7 @@ struct LstmLayerImpl {
     bool forward_done = false;
     int recurrence_mode = 1;   // 0 stepwise, 1 persistent
     bool force_ffma = false;
+    float x_bound = 0.0f;         // > 0: no |entry| of the layer's input exceeds it (the layer stack knows its layers' ranges)
     bool check_padding = false;   // load_sequences verifies that padding frames trail their sequences
     int *pad_dev = nullptr;       // result word of that check
     LstmBuffers bufs{};

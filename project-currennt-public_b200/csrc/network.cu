@@ -118,7 +118,7 @@ int FeedForwardLayer::computeForwardPass(int) {
     {
         ProfScope ps(net_, "ff_forward_gemm");
         // outputs(ls x N) = W^T X with W the pls x ls column-major weight matrix
-        B2_TRY(net_.gemm(outputs_, ls, weights_, pls, 1, prev_->outputs(), 1, pls, ls, N, pls, false));
+        B2_TRY(net_.gemm(outputs_, ls, weights_, pls, 1, prev_->outputs(), 1, pls, ls, N, pls, false, prev_->outputBound()));
     }
     ProfScope ps(net_, "ff_bias_act");
     return ff_bias_act(outputs_, weights_ + (size_t)ls * pls, bias_, ls, (size_t)N * ls, act_, net_.stream);
@@ -138,19 +138,18 @@ int FeedForwardLayer::computeBackwardPass(int) {
         const bool tc = !net_.forceFfma && gemm_wants_tc(1, pls, ls, 1, pls, ls, N) &&
                         (!wantDx || gemm_wants_tc(1, pls, 1, ls, pls, N, ls));
         if (tc) {
-            // both products on the tensor cores: the deltas are split into tf32 hi/lo parts ONCE; the same
-            // [frame][unit] copy serves as the K-major operand of dX and as the MN-major operand of dW
+            // both products on the tensor cores: every operand is split into hi/lo parts ONCE; the deltas' [frame][unit]
+            // copy serves as the K-major operand of dX and as the MN-major operand of dW
             TcScratch &sc = net_.tcScratch;
             B2_TRY(sc.reserve(split_floats(N, ls) + split_floats(N, pls) + split_floats(ls, pls)));
             sc.used = 0;
             SplitOperand sD{}, sX{}, sW{};
-            B2_TRY(split_operand(sc, outputErrors_, ls, N, ls, true, &sD, net_.stream));
-            if (wantDx) {
-                B2_TRY(split_operand(sc, weights_, pls, ls, pls, false, &sW, net_.stream));
+            const SplitJob jobs[3] = {{outputErrors_, ls, N, ls, true, 0.0f, &sD}, {prev_->outputs(), pls, N, pls, false, prev_->outputBound(), &sX},
+                                      {weights_, pls, ls, pls, false, 0.0f, &sW}};
+            B2_TRY(split_operands(sc, jobs, wantDx ? 3 : 2, net_.stream));
+            if (wantDx)
                 B2_TRY(gemm_tc(prev_->outputErrors(), pls, sW, sD, pls, N, ls, false, net_.ws, net_.wsFloats, net_.statusDev,
                                net_.stream));
-            }
-            B2_TRY(split_operand(sc, prev_->outputs(), pls, N, pls, false, &sX, net_.stream));
             SplitOperand sDt = sD;
             sDt.kmajor = false;
             B2_TRY(gemm_tc(weightUpdates_, pls, sX, sDt, pls, ls, N, false, net_.ws, net_.wsFloats, net_.statusDev, net_.stream));
@@ -197,6 +196,7 @@ int LstmLayer::loadSequences(const Fraction &f, int nnState) {
 int LstmLayer::computeForwardPass(int) {
     impl_.force_ffma = net_.forceFfma;
     impl_.recurrence_mode = net_.recurrenceMode;
+    impl_.x_bound = prev_->outputBound();
     return impl_.forward(weights_, prev_->outputs(), outputs_, net_.stream);
 }
 int LstmLayer::computeBackwardPass(int) {
@@ -271,8 +271,8 @@ NeuralNetwork::~NeuralNetwork() {
 }
 
 int NeuralNetwork::gemm(float *C, long ldc, const float *A, long sam, long sak, const float *B, long sbk, long sbn,
-                        int m, int n, int k, bool acc) {
-    return gemm_auto(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, acc, forceFfma, &tcScratch, ws, wsFloats, statusDev, stream);
+                        int m, int n, int k, bool acc, float bBound) {
+    return gemm_auto(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, acc, forceFfma, &tcScratch, ws, wsFloats, statusDev, stream, bBound);
 }
 
 int NeuralNetwork::create(const char *networkJson, int P_, int maxT_, unsigned seed) {
@@ -669,22 +669,20 @@ int b2_matrix_multiply(float *C, int ldc, const float *A, int lda, int transA, c
     Slot &sl = slots[dev];
     std::lock_guard<std::mutex> lk(sl.mu);
     if (!sl.status) {
-        B2_CUDA(cudaMalloc(&sl.status, sizeof(int)));
-        B2_CUDA(cudaMemset(sl.status, 0, sizeof(int)));
+        // the status word lies in host memory the device can write: reading it after the call needs no copy
+        B2_CUDA(cudaHostAlloc((void **)&sl.status, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+        *sl.status = 0;
         B2_CUDA(cudaMalloc(&sl.ws, wsFloats * sizeof(float)));
     }
-    TcScratch &sc = sl.sc;
-    int *status = sl.status;
-    float *ws = sl.ws;
-    B2_TRY(gemm_auto(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, accumulate != 0, force_ffma != 0, &sc, ws, wsFloats, status,
+    volatile int *status = sl.status;
+    B2_TRY(gemm_auto(C, ldc, A, sam, sak, B, sbk, sbn, m, n, k, accumulate != 0, force_ffma != 0, &sl.sc, sl.ws, wsFloats, sl.status,
                      (cudaStream_t)stream));
     if (!force_ffma && gemm_wants_tc(sam, sak, sbk, sbn, m, n, k)) {
         // the arena may be reused by the next call: finish, and report a timed-out wait
-        int v = 0;
-        B2_CUDA(cudaMemcpyAsync(&v, status, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
         B2_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+        const int v = *status;
         if (v != 0) {
-            B2_CUDA(cudaMemset(status, 0, sizeof(int)));
+            *status = 0;
             set_error("b2_matrix_multiply: the tensor-core kernel gave up a bounded wait (status %d)", v);
             return v;
         }

@@ -44,6 +44,7 @@ public:
     const char *patTypes() const { return pat_; }
     Layer *precedingLayer() { return prev_; }
     virtual int loadSequences(const Fraction &f, int nnState);
+    virtual float outputBound() const { return 0.0f; }   // > 0: no output exceeds it in magnitude
     virtual int computeForwardPass(int nnState) = 0;
     virtual int computeBackwardPass(int nnState) = 0;
     int allocate();
@@ -96,6 +97,7 @@ public:
     FeedForwardLayer(NeuralNetwork &net, const json::Value &j, int P, int maxT, Layer *prev, int act);
     int computeForwardPass(int nnState) override;
     int computeBackwardPass(int nnState) override;
+    float outputBound() const override { return act_ == ACT_IDENTITY ? 0.0f : 1.0f; }
 
 private:
     int act_;
@@ -109,6 +111,7 @@ public:
     int loadSequences(const Fraction &f, int nnState) override;
     int computeForwardPass(int nnState) override;
     int computeBackwardPass(int nnState) override;
+    float outputBound() const override { return 1.0f; }   // |tanh(c) * og| < 1
     LstmLayerImpl &impl() { return impl_; }
 
 private:
@@ -205,7 +208,7 @@ public:
     DpComm *dp = nullptr;
     std::vector<cudaEvent_t> gradReady;   // one per layer
     int gemm(float *C, long ldc, const float *A, long sam, long sak, const float *B, long sbk, long sbn, int m, int n,
-             int k, bool acc);
+             int k, bool acc, float bBound = 0.0f);
 
 private:
     unsigned long long profLaunch0_ = 0;
