@@ -208,6 +208,16 @@ bool lstm_single_supported(const LstmShape &s, bool backward);
 int lstm_single_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
                       cudaStream_t st);
 
+// persistent tensor-core recurrence of 513 to 1024 units per direction (lstm_wide.cu).  Returns as above.
+struct WideBuffers {
+    unsigned char *xchg = nullptr;   // operand images and partial sums of a step, two step parities
+    unsigned *flags = nullptr;       // step counters the blocks publish to each other
+};
+bool lstm_wide_supported(const LstmShape &s);
+void lstm_wide_sizes(size_t *exchange_bytes, size_t *flag_words);
+int lstm_wide_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const WideBuffers &wb, const float *w, float *y, const float *dy,
+                    int *status, unsigned *tag_next, cudaStream_t st);
+
 // persistent kernels (lstm_persistent.cu).  Return B2_OK, an error, or 1 when the shape has no
 // persistent kernel (the caller then uses the stepwise kernels).
 bool persistent_geometry(int els, int *JB);   // hidden units per block of the register-resident geometry

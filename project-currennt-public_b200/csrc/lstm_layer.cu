@@ -72,6 +72,8 @@ void LstmLayerImpl::destroy() {
     tcrec = TcRecBuffers();
     cudaFree(ptc.maxbits); cudaFree(ptc.scale); cudaFree(ptc.wimg_f); cudaFree(ptc.wimg_b); cudaFree(ptc.xh); cudaFree(ptc.xe); cudaFree(ptc.flags);
     ptc = PtcBuffers();
+    cudaFree(wide.xchg); cudaFree(wide.flags);
+    wide = WideBuffers();
     if (own_scratch) { own_scratch->release(); delete own_scratch; own_scratch = nullptr; scratch = nullptr; }
     bufs = LstmBuffers();
     ws = nullptr; xchg = nullptr; status_dev = nullptr;
@@ -149,10 +151,16 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
             fwd_path = 5;
             if (rc == 1) ptc_used = false;
         }
-        tcrec_used = !cluster_used && !ptc_used && want_tc_recurrence();
-        const bool plain = !cluster_used && !ptc_used && !tcrec_used;
+        wide_used = !cluster_used && !ptc_used && want_wide();
+        if (wide_used) {
+            B2_TRY(ensure_wide());
+            rc = lstm_wide_sweep(false, s, bufs, wide, w, y, nullptr, status_dev, &tag_next, st);
+            fwd_path = 5;
+        }
+        tcrec_used = !cluster_used && !ptc_used && !wide_used && want_tc_recurrence();
+        const bool plain = !cluster_used && !ptc_used && !wide_used && !tcrec_used;
         if (plain) B2_TRY(lstm_prepare_wrecT(s, w, bufs.wrecT, st));
-        if (cluster_used || ptc_used) {
+        if (cluster_used || ptc_used || wide_used) {
         } else if (tcrec_used) {
             B2_TRY(ensure_tcrec());
             rc = lstm_forward_tc(s, bufs, tcrec, w, y, status_dev, st);
@@ -185,6 +193,9 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
             bwd_path = single ? 1 : 7;
         } else if (ptc_used && recurrence_mode != 6) {
             rc = lstm_ptc_sweep(true, s, bufs, ptc, w, nullptr, dy, status_dev, &tag_next, st);
+            bwd_path = 5;
+        } else if (wide_used) {
+            rc = lstm_wide_sweep(true, s, bufs, wide, w, nullptr, dy, status_dev, &tag_next, st);
             bwd_path = 5;
         }
         if (rc != 1) {
@@ -340,6 +351,29 @@ bool LstmLayerImpl::want_ptc() const {
     if (force_ffma || !lstm_ptc_supported(s)) return false;
     if (recurrence_mode == 5 || recurrence_mode == 6) return true;
     return recurrence_mode == 1 && s.P >= 16;
+}
+
+// The persistent tensor-core kernels of 513 to 1024 units per direction.  Few sequences of 1024 units are left to the FFMA kernels
+// (lstm_persistent.cu), whose step is shorter while one pass of 8 sequences (or one sequence per direction) covers the fraction (B200, us
+// per step forward / backward: one sequence, bidirectional 3.6 / 3.4 there, 4.6 / 5.9 here; unidirectional 1 to 8 sequences 1.8 / 1.7 to
+// 4.9 / 4.8 there, 4.5 / 5.6 here; 2 sequences, bidirectional 9.1 / 9.2 and 4.6 / 5.8).
+bool LstmLayerImpl::want_wide() const {
+    const LstmShape s = shape();
+    if (force_ffma || recurrence_mode != 1 || !lstm_wide_supported(s)) return false;
+    int JB = 0;
+    return !(persistent_geometry(s.els, &JB) && (s.P == 1 || (s.D == 1 && s.P <= 8)));
+}
+
+int LstmLayerImpl::ensure_wide() {
+    if (wide.flags) return B2_OK;
+    size_t xb = 0, nf = 0;
+    lstm_wide_sizes(&xb, &nf);
+    B2_CUDA(cudaMalloc(&wide.xchg, xb));
+    B2_CUDA(cudaMalloc(&wide.flags, nf * sizeof(unsigned)));
+    B2_CUDA(cudaMemset(wide.xchg, 0, xb));
+    B2_CUDA(cudaMemset(wide.flags, 0, nf * sizeof(unsigned)));
+    state_bytes += xb + nf * sizeof(unsigned);
+    return B2_OK;
 }
 
 int LstmLayerImpl::ensure_ptc() {

@@ -35,11 +35,16 @@ struct LstmLayerImpl {
     PtcBuffers ptc{};
     bool ptc_used = false;        // this fraction's forward sweep ran on the persistent tensor-core kernels
     bool cluster_used = false;    // this fraction's forward sweep ran on the register-resident cluster kernels
+    // persistent tensor-core recurrence of wide layers: exchange buffers (allocated on first use)
+    WideBuffers wide{};
+    bool wide_used = false;       // this fraction's forward sweep ran on them
+    bool want_wide() const;
+    int ensure_wide();
     bool want_cluster() const;
     bool want_ptc() const;
     int ensure_ptc();
     // which recurrence the last forward / backward sweep actually ran: 0 one launch per timestep, 1 persistent
-    // FFMA kernels, 3 tensor-core GEMM + gate kernel per timestep, 5 persistent tensor-core kernels, 7 register-resident cluster kernels
+    // FFMA kernels, 3 tensor-core GEMM + gate kernel per timestep, 5 persistent tensor-core kernels (512 units: lstm_ptc.cu, more: lstm_wide.cu), 7 register-resident cluster kernels
     int fwd_path = -1, bwd_path = -1;
     bool want_tc_recurrence() const;
     int ensure_tcrec();

@@ -558,6 +558,28 @@ def test_cluster_recurrence(els, bi, P, T):
             assert np.array_equal(np.asarray(got[key]), np.asarray(again[key])), "not deterministic: " + key
 
 
+@pytest.mark.parametrize("els,bi,P,T", [(513, 1, 2, 5), (1024, 0, 9, 6), (1024, 1, 16, 4), (600, 1, 17, 5), (1023, 1, 33, 4), (640, 0, 33, 7),
+                                        (1024, 1, 65, 4), (776, 0, 130, 3), (1024, 1, 2, 1), (800, 1, 1, 40)])
+def test_wide_recurrence(els, bi, P, T):
+    """The persistent kernels of 513 to 1024 units per direction: every chunk size, several chunks of a group, chunks whose sequences all
+    end early, unit counts that pad a block's units or whole blocks, one step."""
+    from b2lstm import workloads
+    ls = els * (2 if bi else 1)
+    layers = L(("input", 7), ("blstm" if bi else "lstm", ls), ("feedforward_identity", 5), ("sse", 5))
+    lens = np.array(sorted([max(1, T - (p * 7) % (T + 1)) for p in range(P)], reverse=True), np.int32)
+    x, tg = workloads.make_fraction(7, 5, P, lens, 91, 92)
+    w = workloads.make_weights(layers, 93, 0.08)
+    want = run_kind(checker(), layers, P, lens, x, tg, w)
+    paths = {}
+    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0), paths=paths)
+    assert paths[1] == ("persistent_tensor_core", "persistent_tensor_core"), paths
+    parity.compare_run(layers, got, want, "els%d bi%d P%d" % (els, bi, P), lstm_pad_zero_lens=lens)
+    again = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0))
+    for key in got:
+        if key != "launches":
+            assert np.array_equal(np.asarray(got[key]), np.asarray(again[key])), "not deterministic: " + key
+
+
 def test_recurrent_weight_gradient_with_splits_of_whole_slabs():
     """A contraction length (399 frames x 4 sequences) for which the cheapest number of K splits, rounded to whole slabs, would
     leave the last split empty."""
