@@ -18,11 +18,14 @@
 //
 // Kernel.  One 128 x 128 output tile per block, K in slabs of one 128-byte swizzle row (64 halves or
 // 32 floats).  Warp 0 (one lane) feeds a 3-stage shared-memory ring with TMA (cp.async.bulk.tensor.2d,
-// SWIZZLE_128B, no multicast); warps 1 and 10 (one lane each) issue the tcgen05.mma of the main product and
-// of the cross terms (M=128, N=128, K=16 resp. 8; 12 per slab) on shared-memory descriptors and release
-// slots with tcgen05.commit; warps 2-9 (two per tensor-memory lane quarter, half of the tile's columns each)
-// drain the double-buffered main accumulator from TMEM with tcgen05.ld every SEG slabs, add the
-// segments in registers and finally write C.  Operands may be K-major (k
+// SWIZZLE_128B, no multicast); warp 1 (one lane) issues the tcgen05.mma, two per 16 (resp. 8) contraction positions: the hi and lo
+// parts of B follow each other in shared memory, so that a_hi x [b_hi | b_lo] is ONE instruction (M=128, N=256: main products and
+// one cross term side by side), a_lo x b_hi another (N=128, onto the cross columns), and releases slots with tcgen05.commit;
+// warps 2-9 (two per tensor-memory lane quarter, half of the tile's columns each) drain the double-buffered accumulator pair from TMEM
+// with tcgen05.ld every SEG slabs, add the segments in registers and finally write C.
+// What bounds it: shared memory.  A slab costs the tensor core 768 cycles; three N=128 products read 96 KB of operands for it and TMA
+// writes 64 KB, 1280 cycles at 128 bytes per cycle; with the wide instruction the products read 80 KB (1152).
+// B200, 8192 x 64000 x 2048: 6.5 -> 5.9 ms, 1.09 PFLOP/s counting all three products.  Operands may be K-major (k
 // contiguous) or MN-major (m resp. n contiguous); MN-major tiles are fetched as column blocks one
 // swizzle row wide so that they land in the canonical MN-major SWIZZLE_128B layout.  Optional split-K over
 // gridDim.z into scratch (summed by a second kernel in a fixed order).
@@ -42,7 +45,7 @@ constexpr int BM = 128, STAGES = 3;   // the tile's N extent is a template param
 constexpr int TILE_BYTES = BM * 128;                    // 16 KiB: one operand part (hi or lo) of one stage: 128 rows of one swizzle row
 constexpr int STAGE_BYTES = 4 * TILE_BYTES;             // A_hi, A_lo, B_hi, B_lo
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024; // + slack to align the ring to 1024 B
-constexpr int NTHREADS = 352;   // warp 0 TMA, 1 and 10 MMA issue, 2-9 epilogue
+constexpr int NTHREADS = 320;   // warp 0 TMA, 1 MMA issue, 2-9 epilogue
 constexpr int TC_MAX_BATCH = 8;
 // what differs between the two arithmetic modes
 template <bool F16>
@@ -59,7 +62,7 @@ __host__ __device__ __forceinline__ int f16_scale_exp(unsigned maxbits) {
     int e = 13 - ((int)(maxbits >> 23) - 127);          // subnormal maxima (exponent field 0) end at the clamp
     return e < -100 ? -100 : (e > 100 ? 100 : e);
 }
-constexpr int TMEM_COLS = 512;                          // 2 x 128 main accumulator + 2 x 128 cross terms
+constexpr int TMEM_COLS = 512;                          // 2 x (128 main accumulator + 128 cross terms)
 constexpr long long WAIT_CYCLES = 4000000000LL;         // about two seconds
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -176,7 +179,7 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
                    const __grid_constant__ CUtensorMap mapBhi, const __grid_constant__ CUtensorMap mapBlo, TcArgs a) {
     extern __shared__ unsigned char smem_raw[];
     constexpr int BK = Mode<F16>::BK, SEG = Mode<F16>::SEG, MNBOX = Mode<F16>::MNBOX, MNBOX_BYTES = Mode<F16>::MNBOX_BYTES;
-    __shared__ __align__(8) unsigned long long bars[2 * STAGES + 8];
+    __shared__ __align__(8) unsigned long long bars[2 * STAGES + 4];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int fail_s;
 
@@ -185,12 +188,9 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(STAGES + s); };
-    // the main (hi*hi) accumulator is double-buffered in tensor memory and drained every SEG slabs;
-    // the cross-term accumulator is double-buffered over tiles
+    // the accumulators (hi*hi and cross terms) are double-buffered in tensor memory and drained every SEG slabs
     auto big_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * STAGES + b); };
     auto big_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * STAGES + 2 + b); };
-    auto x_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * STAGES + 4 + b); };
-    auto x_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * STAGES + 6 + b); };
 
     // Persistent over work items (m tile fastest, then n tile, then split / batch): barriers and tensor
     // memory are set up once per block, and the epilogue of one tile (global stores from registers)
@@ -199,9 +199,9 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
     const int nkb_full = (a.kchunk + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 2); }   // both issuers release a slot
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(big_full(b), 1); mbar_init(big_empty(b), 8); mbar_init(x_empty(b), 8); mbar_init(x_full(b), 1);
+            mbar_init(big_full(b), 1); mbar_init(big_empty(b), 8);
         }
         fail_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -252,27 +252,25 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
                     }
                     if (a.b_kmajor) {
                         tma_load_2d(base + 2 * TILE_BYTES, &mapBhi, k0 + b_in, n0 + b_out, full_bar(s));
-                        tma_load_2d(base + 3 * TILE_BYTES, &mapBlo, k0 + b_in, n0 + b_out, full_bar(s));
+                        tma_load_2d(base + 2 * TILE_BYTES + BN * 128, &mapBlo, k0 + b_in, n0 + b_out, full_bar(s));
                     } else {
 #pragma unroll
                         for (int b = 0; b < BN / MNBOX; ++b) {
                             tma_load_2d(base + 2 * TILE_BYTES + b * MNBOX_BYTES, &mapBhi, n0 + MNBOX * b + b_in, k0 + b_out, full_bar(s));
-                            tma_load_2d(base + 3 * TILE_BYTES + b * MNBOX_BYTES, &mapBlo, n0 + MNBOX * b + b_in, k0 + b_out, full_bar(s));
+                            tma_load_2d(base + 2 * TILE_BYTES + BN * 128 + b * MNBOX_BYTES, &mapBlo, n0 + MNBOX * b + b_in, k0 + b_out, full_bar(s));
                         }
                     }
                 }
             }
         }
-    } else if (warp == 1 || warp == 10) {
-        // ---------------- MMA issuers: warp 1 the main products (hi*hi), warp 10 the cross terms ----------------
-        // One thread spends about 85 cycles on issuing an MMA of this shape, more than the tensor core needs to run
-        // it; two issuers with accumulators of their own keep the pipe busy and the summation order fixed.
+    } else if (warp == 1) {
+        // ---------------- MMA issue ----------------
         if (lane == 0) {
-            const bool cross = (warp == 10);
             // instruction descriptor: D=f32, A=B=tf32 (format 2) or f16 (format 0), M=128, N=BN, majors per operand
             const uint32_t fmt = F16 ? 0u : 2u;
             const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((a.a_kmajor ? 0u : 1u) << 15) |
                                    ((a.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+            const uint32_t idesc_wide = idesc + ((uint32_t)(BN >> 3) << 17);      // N = 2 BN
             // K-major: rows of 128 B, 8-row groups 1024 B apart (SBO); one MMA advances 32 B inside the row.
             // MN-major, tf32: [k][32 floats] blocks; 32-wide column blocks 4096 B apart (LBO), groups of 4 k-rows
             // 512 B apart (SBO); one MMA (K=8) advances two such groups = 1024 B.
@@ -286,27 +284,23 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
             const uint32_t a_step = a.a_kmajor ? 32u : mn_step, b_step = a.b_kmajor ? 32u : mn_step;
             // Tensor-memory accumulation rounds toward zero, so a long chain drifts linearly with its
             // length.  Two measures keep fp32 accuracy: the cross terms (2^-11 of the main term) get an
-            // accumulator of their own, and the main accumulator is handed to the epilogue warps every
-            // SEG slabs, which add the segments in registers with round-to-nearest.
+            // accumulator of their own, and both are handed to the epilogue warps every SEG slabs, which
+            // add the segments in registers with round-to-nearest.
             bool ok = true;
-            int kbg = 0, gseg = 0, it = 0;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+            int kbg = 0, gseg = 0;
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
                 if (fail_s) break;
                 const int z = item / (a.tiles_m * a.tiles_n);
                 const int zsplit = a.nbatch ? z % a.splits : z;
                 const int kbeg = zsplit * a.kchunk;
                 const int nkb = min(nkb_full, (a.K - kbeg + BK - 1) / BK);
-                const int xb = it & 1;
-                const uint32_t t_small = tmem_base + (uint32_t)(2 * BN + xb * BN);
-                // the cross-term accumulator of two tiles ago must have been read
-                if (cross && !mbar_wait(x_empty(xb), ((uint32_t)(it >> 1) & 1u) ^ 1u)) { fail_s = 1; ok = false; break; }
                 const int nseg = (nkb + SEG - 1) / SEG;
                 for (int seg = 0; seg < nseg && ok; ++seg, ++gseg) {
                     const int buf = gseg & 1;
                     const uint32_t use = (uint32_t)(gseg >> 1);
-                    if (!cross && !mbar_wait(big_empty(buf), (use & 1u) ^ 1u)) { fail_s = 1; ok = false; break; }
+                    if (!mbar_wait(big_empty(buf), (use & 1u) ^ 1u)) { fail_s = 1; ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t t_big = tmem_base + (uint32_t)buf * BN;
+                    const uint32_t t_main = tmem_base + (uint32_t)(buf * 2 * BN), t_cross = t_main + BN;
                     const int kb_end = min(nkb, (seg + 1) * SEG);
                     for (int kb = seg * SEG; kb < kb_end; ++kb, ++kbg) {
                         const int s = kbg % STAGES;
@@ -317,27 +311,21 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
                             const unsigned long long ahi = make_desc(base + kk * a_step, a_lbo, a_sbo, a_lt);
-                            const unsigned long long bhi = make_desc(base + 2 * TILE_BYTES + kk * b_step, b_lbo, b_sbo, b_lt);
-                            if (cross) {
-                                const unsigned long long alo = make_desc(base + TILE_BYTES + kk * a_step, a_lbo, a_sbo, a_lt);
-                                const unsigned long long blo = make_desc(base + 3 * TILE_BYTES + kk * b_step, b_lbo, b_sbo, b_lt);
-                                if (F16) {
-                                    mma_f16(t_small, alo, bhi, idesc, (kb | kk) ? 1u : 0u);
-                                    mma_f16(t_small, ahi, blo, idesc, 1u);
-                                } else {
-                                    mma_tf32(t_small, alo, bhi, idesc, (kb | kk) ? 1u : 0u);
-                                    mma_tf32(t_small, ahi, blo, idesc, 1u);
-                                }
+                            const unsigned long long alo = make_desc(base + TILE_BYTES + kk * a_step, a_lbo, a_sbo, a_lt);
+                            const unsigned long long b = make_desc(base + 2 * TILE_BYTES + kk * b_step, b_lbo, b_sbo, b_lt);
+                            const uint32_t acc = (kb != seg * SEG || kk) ? 1u : 0u;
+                            if (F16) {
+                                mma_f16(t_main, ahi, b, idesc_wide, acc);
+                                mma_f16(t_cross, alo, b, idesc, 1u);
                             } else {
-                                if (F16) mma_f16(t_big, ahi, bhi, idesc, (kb != seg * SEG || kk) ? 1u : 0u);
-                                else mma_tf32(t_big, ahi, bhi, idesc, (kb != seg * SEG || kk) ? 1u : 0u);
+                                mma_tf32(t_main, ahi, b, idesc_wide, acc);
+                                mma_tf32(t_cross, alo, b, idesc, 1u);
                             }
                         }
-                        mma_commit(empty_bar(s));   // slot is free once both issuers' MMAs have read it
+                        mma_commit(empty_bar(s));   // slot is free once its MMAs have read it
                     }
-                    if (!cross) mma_commit(big_full(buf));   // the main products of this segment are complete
+                    mma_commit(big_full(buf));      // the products of this segment are complete
                 }
-                if (cross && ok) mma_commit(x_full(xb));     // the cross terms of this tile are complete
             }
         }
     } else {
@@ -349,15 +337,14 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
         const int cbase = ((warp - 2) >> 2) * HN;
         const uint32_t lane_base = tmem_base + ((uint32_t)(32 * q) << 16);
         bool ok = true;
-        int gseg = 0, it = 0;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+        int gseg = 0;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
             if (fail_s) break;
             const int m0 = (item % a.tiles_m) * BM, n0 = ((item / a.tiles_m) % a.tiles_n) * BN;
             const int z = item / (a.tiles_m * a.tiles_n);
             const int zsplit = a.nbatch ? z % a.splits : z, batch = a.nbatch ? z / a.splits : 0;
             const int kbeg = zsplit * a.kchunk;
             const int nkb = min(nkb_full, (a.K - kbeg + BK - 1) / BK);
-            const int xb = it & 1;
             float acc[HN];
 #pragma unroll
             for (int j = 0; j < HN; ++j) acc[j] = 0.0f;
@@ -370,11 +357,12 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int c0 = 0; c0 < HN; c0 += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(lane_base + (uint32_t)(buf * BN + cbase + c0), r);
+                    uint32_t r[32], x[32];
+                    tmem_ld32(lane_base + (uint32_t)(buf * 2 * BN + cbase + c0), r);
+                    tmem_ld32(lane_base + (uint32_t)(buf * 2 * BN + BN + cbase + c0), x);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) acc[c0 + j] += __uint_as_float(r[j]);
+                    for (int j = 0; j < 32; ++j) acc[c0 + j] += fmaf(__uint_as_float(x[j]), F16 ? LO_UNSCALE : 1.0f, __uint_as_float(r[j]));
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(big_empty(buf)) : "memory");
@@ -383,25 +371,6 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
                 if (lane == 0) fail_s = 1;
                 break;
             }
-            // the cross terms; after this read tensor memory is free for the tile after next, and the stores
-            // below run under the next tile's MMAs
-            ok = __all_sync(0xffffffffu, mbar_wait(x_full(xb), (uint32_t)(it >> 1) & 1u));
-            if (!ok) {
-                if (lane == 0) fail_s = 1;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int c0 = 0; c0 < HN; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32(lane_base + (uint32_t)(2 * BN + xb * BN + cbase + c0), r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < 32; ++j) acc[c0 + j] += F16 ? __uint_as_float(r[j]) * LO_UNSCALE : __uint_as_float(r[j]);
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(x_empty(xb)) : "memory");
-
             // fp16 mode: undo the operand scales (two exact factors: their product may leave the fp32 range)
             float inv_a = 1.0f, inv_b = 1.0f;
             if (F16) { inv_a = ldexpf(1.0f, -f16_scale_exp(*a.a_max)); inv_b = ldexpf(1.0f, -f16_scale_exp(*a.b_max)); }
