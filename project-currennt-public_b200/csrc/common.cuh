@@ -88,11 +88,17 @@ size_t split_floats(int outer, int inner);
 int split_tf32(const float *src, long s_outer, int outer, int inner, float *hi, float *lo, long ldp, cudaStream_t st);
 // One operand to be split into fp16 parts: `outer` rows of `inner` contiguous entries, rows s_outer floats apart.  bound > 0: the
 // caller's promise that no |entry| exceeds it (saves the pass that finds the largest entry).  *out receives the parts.
-struct SplitJob { const float *src; long s_outer; int outer, inner; bool kmajor; float bound; SplitOperand *out; };
+// map: the rows of src to take (NULL: all of them in their order).  shift: columns below shift_cols come from the row `shift` below the
+// mapped one, the others from the row `shift` above; zeros where src (src_rows rows) has none.
+struct SplitJob {
+    const float *src; long s_outer; int outer, inner; bool kmajor; float bound; SplitOperand *out;
+    const int *map = nullptr;
+    int shift = 0, shift_cols = 0, src_rows = 0;
+};
 int split_operands(TcScratch &sc, const SplitJob *jobs, int n, cudaStream_t st);
 bool gemm_tc_supported(const SplitOperand &A, const SplitOperand &B, int m, int n, int k);
 int gemm_tc(float *C, long ldc, const SplitOperand &A, const SplitOperand &B, int m, int n, int k, bool accumulate,
-            float *ws, size_t ws_floats, int *status, cudaStream_t st);
+            float *ws, size_t ws_floats, int *status, cudaStream_t st, const int *n_map = nullptr);   // n_map: column of C of every n
 // Planned, batched launches of the tensor-core kernel: tensor maps encoded once, many launches that
 // differ in coordinate offsets.  Batch b shifts operand A by (a_in, a_out) and B by (b_in, b_out) in
 // (contiguous index, other index) coordinates and writes split z to C + c_off + z*c_split_stride.
@@ -133,6 +139,10 @@ int sgd_update(float *w, float *g, float *delta, size_t n, float lr, float mom, 
 // accumulates the AdaGrad statistics, 5 Adam; stats holds n floats (2n for Adam)
 int sgd_update_opt(float *w, float *g, float *delta, float *stats, size_t n, float lr, float mom, int option,
                    const float *frac_len_dev, float beta1_accum, float beta2_accum, cudaStream_t st);
+// pattern types and list of the real frames of a fraction from its sequence lengths (lens: P lengths, P running sums, on the device)
+int fraction_maps(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st);
+// zeroes the rows of m(frames x cols) that belong to padding frames
+int zero_padding_rows(float *m, int cols, const char *pat, int frames, cudaStream_t st);
 int fill_value(float *p, size_t n, float v, cudaStream_t st);
 // acc = g (first) or acc + g
 int accumulate(float *acc, const float *g, size_t n, bool first, cudaStream_t st);
@@ -151,6 +161,8 @@ struct LstmBuffers {
     float *cerr;        // [2][P][ls]:  cell-state errors of the two most recent steps (stepwise kernels)
     float *wrecT;       // [D][els][4][els]: recurrent weights, source unit major (forward sweep)
     const char *pat;    // [T*P]
+    const int *real = nullptr;   // the real frames of the fraction, n_real of them (NULL: take all frames)
+    int n_real = 0;
 };
 // one launch per timestep, both directions in the same launch
 int lstm_forward_stepwise(const LstmShape &s, const LstmBuffers &b, const float *w, float *y, cudaStream_t st);

@@ -269,6 +269,35 @@ int accumulate(float *acc, const float *g, size_t n, bool first, cudaStream_t st
     return B2_OK;
 }
 
+// Pattern types of a fraction (1 first, 2 inner, 3 last frame of a sequence, 0 padding) and the list of its real frames, sequence by
+// sequence; one thread per frame.  lens[0..P) are the lengths, lens[P..2P) their running sums.
+namespace {
+__global__ void fraction_kernel(const int *__restrict__ lens, int P, int frames, char *__restrict__ pat, int *__restrict__ map) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= frames) return;
+    const int t = f / P, p = f - t * P, len = __ldg(lens + p);
+    pat[f] = t >= len ? PAT_NONE : (t == 0 ? 1 : (t == len - 1 ? 3 : 2));
+    if (t < len) map[__ldg(lens + P + p) + t] = f;
+}
+__global__ void zero_padding_kernel(float *__restrict__ m, int cols, const char *__restrict__ pat, int frames) {
+    for (int f = blockIdx.x * 8 + (int)(threadIdx.x >> 5); f < frames; f += gridDim.x * 8)
+        if (pat[f] == PAT_NONE)
+            for (int c = threadIdx.x & 31; c < cols; c += 32) m[(size_t)f * cols + c] = 0.0f;
+}
+}  // namespace
+int fraction_maps(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st) {
+    fraction_kernel<<<(frames + 255) / 256, 256, 0, st>>>(lens, P, frames, pat, map);
+    count_launch();
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+int zero_padding_rows(float *m, int cols, const char *pat, int frames, cudaStream_t st) {
+    const int want = (frames + 7) / 8, most = sm_count() * 8;
+    zero_padding_kernel<<<want < most ? want : most, 256, 0, st>>>(m, cols, pat, frames);
+    count_launch();
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
 int fill_value(float *p, size_t n, float v, cudaStream_t st) {
     if (!n) return B2_OK;
     fill_value_kernel<<<grid_for(n, 256), 256, 0, st>>>(p, n, v);

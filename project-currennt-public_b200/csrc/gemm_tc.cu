@@ -171,6 +171,7 @@ struct TcArgs {
     int kseg_len, kseg_stride;
     // work items of the persistent tile loop: tiles_m x tiles_n output tiles x nz splits / batches
     int tiles_m, tiles_n, nz;
+    const int *n_map;  // column of C that row n of B belongs to (NULL: n)
 };
 
 template <int BN, bool F16>
@@ -380,17 +381,26 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
             float *dst = batched ? a.C + a.c_off[batch] + (long long)zsplit * a.c_split_stride
                                  : (split ? a.ws + (size_t)z * (size_t)a.M * a.N : a.C);
             const long ld = split ? (long)a.M : a.ldc;
-            if (m < a.M) {
+            auto store = [&](int j, int col) {
+                float *p = dst + (size_t)col * ld + m;
+                float v = F16 ? acc[j] * inv_a * inv_b : acc[j];
+                if (!split && !batched && a.accumulate) v += *p;
+                *p = v;
+            };
+            if (a.n_map && !split) {
+                // lane l holds the columns of C for rows l and l + 32 of this warp's part of B
+                int col[2];
+#pragma unroll
+                for (int h = 0; h < HN / 32; ++h) col[h] = n0 + cbase + 32 * h + lane < a.N ? __ldg(a.n_map + n0 + cbase + 32 * h + lane) : 0;
 #pragma unroll
                 for (int j = 0; j < HN; ++j) {
-                    const int n = n0 + cbase + j;
-                    if (n < a.N) {
-                        float *p = dst + (size_t)n * ld + m;
-                        float v = F16 ? acc[j] * inv_a * inv_b : acc[j];
-                        if (!split && !batched && a.accumulate) v += *p;
-                        *p = v;
-                    }
+                    const int c = __shfl_sync(0xffffffffu, col[j / 32], j % 32);
+                    if (m < a.M && n0 + cbase + j < a.N) store(j, c);
                 }
+            } else if (m < a.M) {
+#pragma unroll
+                for (int j = 0; j < HN; ++j)
+                    if (n0 + cbase + j < a.N) store(j, n0 + cbase + j);
             }
         }
     }
@@ -403,13 +413,13 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_cons
 }
 
 __global__ void tc_splitk_reduce_kernel(float *__restrict__ C, long ldc, const float *__restrict__ ws, int M, int N,
-                                        int splits, int accumulate) {
+                                        int splits, int accumulate, const int *__restrict__ n_map) {
     size_t total = (size_t)M * N;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         float s = 0.0f;
         for (int z = 0; z < splits; ++z) s += ws[(size_t)z * total + i];
         size_t m = i % M, n = i / M;
-        float *p = C + n * ldc + m;
+        float *p = C + (n_map ? (size_t)__ldg(n_map + n) : n) * ldc + m;
         *p = accumulate ? *p + s : s;
     }
 }
@@ -502,6 +512,8 @@ struct SplitWork {
     unsigned *maxbits;         // receives the bit pattern the scale follows from
     unsigned *partial;         // the blocks' maxima
     int vec, parts;            // 16-byte accesses possible; blocks (= partial results)
+    const int *map;            // as in SplitJob
+    int shift, shift_cols, src_rows;
 };
 struct SplitBatch { SplitWork w[MAX_SPLIT_JOBS]; int first[MAX_SPLIT_JOBS + 1]; };   // first block of each job
 
@@ -535,19 +547,19 @@ __global__ void __launch_bounds__(256) absmax_batch_kernel(const __grid_constant
     if (w.vec) {
         const unsigned in4 = (unsigned)w.inner / 4;
         const size_t total = (size_t)w.outer * in4;
-        const bool dense = w.s_outer == w.inner;
+        const bool dense = w.s_outer == w.inner && !w.map;
         for (size_t i = i0; i < total; i += stride) {
-            const float4 x = __ldg(dense ? (const float4 *)w.src + i : (const float4 *)(w.src + (i / in4) * w.s_outer) + i % in4);
+            const float4 x = __ldg(dense ? (const float4 *)w.src + i : (const float4 *)(w.src + (size_t)(w.map ? __ldg(w.map + i / in4) : i / in4) * w.s_outer) + i % in4);
             m = max(m, max(max(finite_bits(x.x), finite_bits(x.y)), max(finite_bits(x.z), finite_bits(x.w))));
         }
-    } else if (w.s_outer == w.inner) {
+    } else if (w.s_outer == w.inner && !w.map) {
         const size_t total = (size_t)w.outer * w.inner;
 #pragma unroll 4
         for (size_t i = i0; i < total; i += stride) m = max(m, finite_bits(__ldg(w.src + i)));
     } else {
         // a warp per row
         for (int r = block * 8 + (int)(threadIdx.x >> 5); r < w.outer; r += w.parts * 8)
-            for (int c = threadIdx.x & 31; c < w.inner; c += 32) m = max(m, finite_bits(__ldg(w.src + (size_t)r * w.s_outer + c)));
+            for (int c = threadIdx.x & 31; c < w.inner; c += 32) m = max(m, finite_bits(__ldg(w.src + (size_t)(w.map ? __ldg(w.map + r) : r) * w.s_outer + c)));
     }
     m = block_max256(m);
     if (threadIdx.x == 0) w.partial[block] = m;
@@ -576,9 +588,14 @@ __global__ void __launch_bounds__(256) split_f16_batch_kernel(const __grid_const
     const size_t total = (size_t)w.outer * ld8;
     for (size_t i = (size_t)block * 256 + threadIdx.x; i < total; i += (size_t)w.parts * 256) {
         const unsigned r = total <= 0xffffffffu ? (unsigned)i / ld8 : (unsigned)(i / ld8), c = (unsigned)(i - (size_t)r * ld8) * 8u;
-        const float *p = w.src + (size_t)r * w.s_outer + c;
+        long row = w.map ? (long)__ldg(w.map + r) : (long)r;
+        if (w.shift) row += c < (unsigned)w.shift_cols ? -w.shift : w.shift;
+        const float *p = w.src + row * w.s_outer + c;
         float in[8];
-        if (w.vec) {
+        if (w.shift && (row < 0 || row >= w.src_rows)) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) in[e] = 0.0f;
+        } else if (w.vec) {
             const float4 x0 = __ldg((const float4 *)p), x1 = c + 4 < (unsigned)w.inner ? __ldg((const float4 *)p + 1) : make_float4(0, 0, 0, 0);
             in[0] = x0.x; in[1] = x0.y; in[2] = x0.z; in[3] = x0.w; in[4] = x1.x; in[5] = x1.y; in[6] = x1.z; in[7] = x1.w;
         } else {
@@ -700,6 +717,7 @@ int split_operands(TcScratch &sc, const SplitJob *jobs, int n, cudaStream_t st) 
         if (!hi || !lo || !mb) { set_error("split_operands: operand arena exhausted"); return B2_ERR_BAD_SHAPE; }
         w.src = q.src; w.s_outer = q.s_outer; w.outer = q.outer; w.inner = q.inner;
         w.hi = (unsigned short *)hi; w.lo = (unsigned short *)lo;
+        w.map = q.map; w.shift = q.shift; w.shift_cols = q.shift_cols; w.src_rows = q.src_rows;
         w.bound = q.bound > 0.0f ? float_bits(q.bound) : 0u;
         w.maxbits = (unsigned *)mb; w.partial = (unsigned *)mb + 64;
         w.vec = (q.inner % 4) == 0 && (q.s_outer % 4) == 0 && ((uintptr_t)q.src % 16) == 0;
@@ -736,7 +754,7 @@ bool gemm_tc_supported(const SplitOperand &A, const SplitOperand &B, int m, int 
 // C(m x n) (+)= A' B' from pre-split operands.  K-major A: rows m, `ld` floats apart, k contiguous;
 // MN-major A: rows k, m contiguous.  Likewise B with n.
 int gemm_tc(float *C, long ldc, const SplitOperand &A, const SplitOperand &B, int m, int n, int k, bool accumulate, float *ws,
-            size_t ws_floats, int *status, cudaStream_t st) {
+            size_t ws_floats, int *status, cudaStream_t st, const int *n_map) {
     B2_TRY(get_encode());
     B2_TRY(set_kernel_attributes());
     if (!gemm_tc_supported(A, B, m, n, k)) { set_error("gemm_tc: operand parts missing, misaligned or of different kinds"); return B2_ERR_BAD_ARG; }
@@ -776,19 +794,19 @@ int gemm_tc(float *C, long ldc, const SplitOperand &A, const SplitOperand &B, in
     kchunk = (kchunk + BK - 1) / BK * BK;
     splits = (k + kchunk - 1) / kchunk;
     grid.z = splits;
-    TcArgs a;
+    TcArgs a{};
     a.C = C; a.ldc = ldc; a.M = m; a.N = n; a.K = k; a.kchunk = kchunk;
     a.a_kmajor = A.kmajor ? 1 : 0; a.b_kmajor = B.kmajor ? 1 : 0;
     a.accumulate = accumulate ? 1 : 0; a.ws = ws; a.status = status;
     a.a_max = A.maxbits; a.b_max = B.maxbits;
     a.nbatch = 0; a.splits = splits; a.c_split_stride = 0; a.kseg_len = 0; a.kseg_stride = 0;
-    a.tiles_m = (int)grid.x; a.tiles_n = (int)grid.y; a.nz = splits;
+    a.tiles_m = (int)grid.x; a.tiles_n = (int)grid.y; a.nz = splits; a.n_map = n_map;
     B2_TRY(launch_kernel(BN, f16, persistent_grid(a.tiles_m * a.tiles_n * a.nz), mAh, mAl, mBh, mBl, a, st));
     if (splits > 1) {
         size_t total = (size_t)m * n;
         int blocks = (int)((total + 255) / 256);
         if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-        tc_splitk_reduce_kernel<<<blocks, 256, 0, st>>>(C, ldc, ws, m, n, splits, accumulate ? 1 : 0);
+        tc_splitk_reduce_kernel<<<blocks, 256, 0, st>>>(C, ldc, ws, m, n, splits, accumulate ? 1 : 0, n_map);
         count_launch();
         B2_CUDA(cudaGetLastError());
     }

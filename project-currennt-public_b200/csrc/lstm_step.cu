@@ -213,11 +213,12 @@ __global__ void lstm_vgrad_partial_kernel(LstmShape sh, LstmBuffers bf, float *_
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= ls) return;
     const int d = u / els;
-    const long N = (long)sh.T * P;
-    long f0 = (long)blockIdx.y * frames_per_chunk, f1 = min(N, f0 + frames_per_chunk);
+    const long N = (long)sh.T * P, frames = bf.real ? bf.n_real : N;      // padding frames add nothing
+    const long i0 = (long)blockIdx.y * frames_per_chunk, i1 = min(frames, i0 + frames_per_chunk);
     float s[7] = {0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
-    for (long f = f0; f < f1; ++f) {
+    for (long i = i0; i < i1; ++i) {
+        const long f = bf.real ? __ldg(bf.real + i) : i;
         const float *dl = bf.deltas + (size_t)f * 4 * ls + u;
         float dni = dl[0], dig = dl[ls], dfg = dl[2 * ls], dog = dl[3 * ls];
         s[0] += dni; s[1] += dig; s[2] += dfg; s[3] += dog;
@@ -285,7 +286,7 @@ int lstm_backward_stepwise(const LstmShape &s, const LstmBuffers &b, const float
 
 int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, float *dw, float *ws, size_t ws_floats,
                       cudaStream_t st) {
-    long N = (long)s.T * s.P;
+    const long N = b.real ? b.n_real : (long)s.T * s.P;
     // chunks of frames: enough blocks to fill the device several times over, bounded by the scratch
     int fpc = 64;
     const long max_chunks = (long)(ws_floats / ((size_t)7 * s.ls));

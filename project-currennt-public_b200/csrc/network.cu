@@ -191,7 +191,9 @@ int LstmLayer::init() {
 }
 int LstmLayer::loadSequences(const Fraction &f, int nnState) {
     Layer::loadSequences(f, nnState);
-    return impl_.load_sequences(f.T, f.Tmin, f.patTypes);
+    B2_TRY(impl_.load_sequences(f.T, f.Tmin, f.patTypes));
+    impl_.set_real_frames(f.realMap, (int)f.realFrames);
+    return B2_OK;
 }
 int LstmLayer::computeForwardPass(int) {
     impl_.force_ffma = net_.forceFfma;
@@ -255,8 +257,8 @@ NeuralNetwork::~NeuralNetwork() {
     layers.clear();
     cudaFree(ws); cudaFree(statusDev); cudaFree(fracLenDev);
     for (int b = 0; b < 2; ++b) {
-        cudaFree(inBuf[b]); cudaFree(tgBuf[b]); cudaFree(patBuf[b]);
-        if (patPinned[b]) cudaFreeHost(patPinned[b]);
+        cudaFree(inBuf[b]); cudaFree(tgBuf[b]); cudaFree(patBuf[b]); cudaFree(mapBuf[b]); cudaFree(lenBuf[b]);
+        if (lenPinned[b]) cudaFreeHost(lenPinned[b]);
         if (prefetchDone[b]) cudaEventDestroy(prefetchDone[b]);
         if (bufFree[b]) cudaEventDestroy(bufFree[b]);
         if (patCopied[b]) cudaEventDestroy(patCopied[b]);
@@ -343,7 +345,9 @@ int NeuralNetwork::create(const char *networkJson, int P_, int maxT_, unsigned s
         B2_CUDA(cudaMalloc(&inBuf[b], frames * layers.front()->size() * sizeof(float)));
         B2_CUDA(cudaMalloc(&tgBuf[b], frames * layers.back()->size() * sizeof(float)));
         B2_CUDA(cudaMalloc(&patBuf[b], frames));
-        B2_CUDA(cudaMallocHost(&patPinned[b], frames));
+        B2_CUDA(cudaMalloc(&mapBuf[b], frames * sizeof(int)));
+        B2_CUDA(cudaMalloc(&lenBuf[b], (size_t)2 * P * sizeof(int)));
+        B2_CUDA(cudaMallocHost(&lenPinned[b], (size_t)2 * P * sizeof(int)));
         B2_CUDA(cudaEventCreateWithFlags(&prefetchDone[b], cudaEventDisableTiming));
         B2_CUDA(cudaEventCreateWithFlags(&bufFree[b], cudaEventDisableTiming));
         B2_CUDA(cudaEventCreateWithFlags(&patCopied[b], cudaEventDisableTiming));
@@ -418,20 +422,23 @@ int NeuralNetwork::stageFraction(int b, int T, int nSeq, const int *lens, const 
     }
     // pattern types as DataSet::_makeFractionTask writes them (data_sets/DataSet.cpp:853-861)
     size_t frames = (size_t)mx * P;
-    char *ph = patPinned[b];
+    int *lh = lenPinned[b];
     // the pinned staging is rewritten by the host: the previous copy out of it must have run
     B2_CUDA(cudaEventSynchronize(patCopied[b]));
-    memset(ph, 0, frames);
-    for (int p = 0; p < nSeq; ++p)
-        for (int t = 0; t < lens[p]; ++t) ph[(size_t)t * P + p] = t == 0 ? 1 : (t == lens[p] - 1 ? 3 : 2);
-    B2_CUDA(cudaMemcpyAsync(patBuf[b], ph, frames, cudaMemcpyHostToDevice, st));
+    for (int p = 0, sum = 0; p < P; ++p) {
+        lh[p] = p < nSeq ? lens[p] : 0;
+        lh[P + p] = sum;
+        sum += lh[p];
+    }
+    B2_CUDA(cudaMemcpyAsync(lenBuf[b], lh, (size_t)2 * P * sizeof(int), cudaMemcpyHostToDevice, st));
     B2_CUDA(cudaEventRecord(patCopied[b], st));
+    B2_TRY(fraction_maps(lenBuf[b], P, (int)frames, patBuf[b], mapBuf[b], st));
     cudaMemcpyKind kind = onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     B2_CUDA(cudaMemcpyAsync(inBuf[b], in, frames * layers.front()->size() * sizeof(float), kind, st));
     B2_CUDA(cudaMemcpyAsync(tgBuf[b], tg, frames * layers.back()->size() * sizeof(float), kind, st));
     Fraction &f = fracBuf[b];
     f.T = mx; f.Tmin = mn; f.nSeq = nSeq; f.realFrames = real;
-    f.patTypes = patBuf[b]; f.inputs = inBuf[b]; f.targets = tgBuf[b];
+    f.patTypes = patBuf[b]; f.realMap = mapBuf[b]; f.inputs = inBuf[b]; f.targets = tgBuf[b];
     return B2_OK;
 }
 

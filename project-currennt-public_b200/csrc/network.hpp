@@ -24,6 +24,7 @@ struct Fraction {
     int T = 0, Tmin = 0, nSeq = 0;
     long realFrames = 0;
     const char *patTypes = nullptr;   // device
+    const int *realMap = nullptr;     // device: frame numbers of the real frames
     const float *inputs = nullptr;    // device, [T*P*inputSize]
     const float *targets = nullptr;   // device, [T*P*outputSize]
 };
@@ -187,7 +188,9 @@ public:
     // (on copyStream) while the current one is being processed
     float *inBuf[2] = {nullptr, nullptr}, *tgBuf[2] = {nullptr, nullptr};
     char *patBuf[2] = {nullptr, nullptr};
-    char *patPinned[2] = {nullptr, nullptr};   // pinned host staging of the pattern types
+    int *mapBuf[2] = {nullptr, nullptr};       // the real frames of the fraction
+    int *lenBuf[2] = {nullptr, nullptr};       // sequence lengths and their running sums
+    int *lenPinned[2] = {nullptr, nullptr};    // ... pinned host staging
     Fraction fracBuf[2];
     int cur = 0;
     bool prefetchPending = false;

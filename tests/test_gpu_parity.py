@@ -580,6 +580,27 @@ def test_wide_recurrence(els, bi, P, T):
             assert np.array_equal(np.asarray(got[key]), np.asarray(again[key])), "not deterministic: " + key
 
 
+@pytest.mark.parametrize("els,bi,P,T,lo,ff", [(64, 1, 9, 60, 1, 0), (72, 0, 17, 70, 3, 40), (128, 1, 32, 40, 20, 24), (100, 1, 5, 90, 1, 33),
+                                              (256, 0, 3, 300, 2, 0), (600, 1, 20, 13, 1, 30)])
+def test_products_without_padding_frames(els, bi, P, T, lo, ff):
+    """Ragged fractions whose products run over the list of real frames: operand gathers, the shifted gather of the recurrent weight
+    gradient (tensor-core and FFMA unit counts), results scattered back, zeros at the padding frames below a feed-forward layer."""
+    from b2lstm import workloads
+    ls = els * (2 if bi else 1)
+    kind = "blstm" if bi else "lstm"
+    spec = [("input", 70)] + ([("feedforward_tanh", ff)] if ff else []) + [(kind, ls), (kind, ls), ("feedforward_identity", 9), ("sse", 9)]
+    layers = L(*spec)
+    r = np.random.RandomState(els)
+    lens = r.randint(lo, T + 1, P).astype(np.int32)      # in no order
+    lens[P // 2], lens[-1] = T, lo
+    x, tg = workloads.make_fraction(70, 9, P, lens, 95, 96)
+    w = workloads.make_weights(layers, 97, 0.08)
+    want = run_kind(checker(), layers, P, lens, x, tg, w)
+    for variant in (dict(recurrence=1, ffma=0), dict(recurrence=1, ffma=1)):
+        got = run_gpu(layers, P, lens, x, tg, w, variant)
+        parity.compare_run(layers, got, want, "els%d bi%d P%d %s" % (els, bi, P, variant), lstm_pad_zero_lens=lens)
+
+
 def test_recurrent_weight_gradient_with_splits_of_whole_slabs():
     """A contraction length (399 frames x 4 sequences) for which the cheapest number of K splits, rounded to whole slabs, would
     leave the last split empty."""
