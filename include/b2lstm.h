@@ -133,8 +133,7 @@ int b2_lstm_backward(b2_lstm *layer, const float *weights_dev, const float *x_de
 int b2_lstm_set_recurrence_mode(b2_lstm *layer, int mode);
 /* Which recurrence kernels the layer's last forward (backward = 0) or backward (backward != 0) sweep really
  * ran, whatever the mode asked for: 0 one launch per timestep, 1 persistent FFMA kernels, 3 tensor-core GEMM
- * and gate kernel per timestep, 5 persistent tensor-core kernels (512 units per direction, or 513 to
- * 1024), 7 tensor-core kernels with register-resident weights on
+ * and gate kernel per timestep, 5 persistent tensor-core kernels, 7 tensor-core kernels with register-resident weights on
  * thread-block clusters; -1 before the first sweep.  The reference
  * has one code path (layers/LstmLayer.cu:1805-1858), so it has no such query. */
 int b2_lstm_recurrence_path(const b2_lstm *layer, int backward);

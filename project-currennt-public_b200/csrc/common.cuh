@@ -211,6 +211,7 @@ int lstm_ptc_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, cons
 // register-resident tensor-core recurrence on thread-block clusters (lstm_cluster.cu): up to 512 units per direction, any number
 // of sequences.  Returns B2_OK, an error, or 1 when no cluster of the needed size fits on the device.
 bool lstm_cluster_supported(const LstmShape &s);
+double lstm_cluster_step_us(const LstmShape &s);   // estimate: a step of the forward sweep and one of the backward sweep
 int lstm_cluster_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
                        cudaStream_t st);
 
@@ -220,13 +221,14 @@ bool lstm_single_supported(const LstmShape &s, bool backward);
 int lstm_single_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
                       cudaStream_t st);
 
-// persistent tensor-core recurrence of 513 to 1024 units per direction (lstm_wide.cu).  Returns as above.
+// persistent tensor-core recurrence of 257 to 1024 units per direction (lstm_wide.cu).  Returns as above.
 struct WideBuffers {
     unsigned char *xchg = nullptr;   // operand images and partial sums of a step, two step parities
     unsigned *flags = nullptr;       // step counters the blocks publish to each other
 };
 bool lstm_wide_supported(const LstmShape &s);
-void lstm_wide_sizes(size_t *exchange_bytes, size_t *flag_words);
+double lstm_wide_step_us(const LstmShape &s);
+void lstm_wide_sizes(const LstmShape &s, size_t *exchange_bytes, size_t *flag_words);
 int lstm_wide_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const WideBuffers &wb, const float *w, float *y, const float *dy,
                     int *status, unsigned *tag_next, cudaStream_t st);
 

@@ -713,9 +713,9 @@ double step_cycles(const Variant &v, int KP, int nt, double share, bool backward
     return first + (nt - 1) * ((mma > packets ? mma : packets) + 400.0);
 }
 
-struct Plan { int vi, nt, items, clusters; };
+struct Plan { int vi, nt, items, clusters; double cycles; };
 Plan make_plan(const LstmShape &s, bool backward) {
-    Plan best{-1, 0, 0, 0};
+    Plan best{-1, 0, 0, 0, 0.0};
     double best_t = 0.0;
     const int tiles = (s.P + 7) / 8;
     for (int vi = 0; vi < (backward ? NBWD : NFWD); ++vi) {
@@ -731,7 +731,7 @@ Plan make_plan(const LstmShape &s, bool backward) {
             const double share = (double)((live + alone - 1) / alone);
             // where two come out equal, the one on fewer SMs: another net's kernels may want the rest
             const double t = passes * step_cycles(v, KP, nt, share, backward) * (1.0 + 0.05 * live * v.C / sm_count());
-            if (best.vi < 0 || t < best_t) { best = Plan{vi, nt, items, live}; best_t = t; }
+            if (best.vi < 0 || t < best_t) { best = Plan{vi, nt, items, live, passes * step_cycles(v, KP, nt, share, backward)}; best_t = t; }
         }
     }
     return best;
@@ -740,6 +740,13 @@ Plan make_plan(const LstmShape &s, bool backward) {
 }  // namespace
 
 bool lstm_cluster_supported(const LstmShape &s) { return s.els <= 512 && make_plan(s, false).vi >= 0 && make_plan(s, true).vi >= 0; }
+
+// The fit of step_cycles holds up to 256 units; beyond, several tiles in turn and 16 blocks a cluster, measured steps are 1.4 times as long
+// (us per step, forward + backward, estimated and measured: 512 units, 64 sequences, bidirectional 7.8 and 11.5, 32 sequences 5.9 and
+// 7.9; 400 units, 128 sequences 15.7 and 23.8; 300 units, 64 sequences 6.5 and 8.8).
+double lstm_cluster_step_us(const LstmShape &s) {
+    return (s.els > 256 ? 1.4 : 1.0) * (make_plan(s, false).cycles + make_plan(s, true).cycles) / 1950.0;
+}
 
 int lstm_cluster_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const float *w, float *y, const float *dy, int *status,
                        cudaStream_t st) {

@@ -162,7 +162,8 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
                         : lstm_cluster_sweep(false, s, bufs, w, y, nullptr, status_dev, st);
             fwd_path = single ? 1 : 7;
         }
-        ptc_used = !cluster_used && want_ptc();
+        wide_used = !cluster_used && want_wide();
+        ptc_used = !cluster_used && !wide_used && want_ptc();
         if (ptc_used) {
             B2_TRY(ensure_ptc());
             B2_TRY(lstm_ptc_prepare(s, w, ptc, st));
@@ -170,7 +171,6 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
             fwd_path = 5;
             if (rc == 1) ptc_used = false;
         }
-        wide_used = !cluster_used && !ptc_used && want_wide();
         if (wide_used) {
             B2_TRY(ensure_wide());
             rc = lstm_wide_sweep(false, s, bufs, wide, w, y, nullptr, status_dev, &tag_next, st);
@@ -354,19 +354,15 @@ bool LstmLayerImpl::want_tc_recurrence() const {
     return passes * (1.4 + 0.27 * ps) > 12.0;
 }
 
-// The register-resident cluster kernels serve up to 512 units per direction (what the registers and tensor memory of 16 SMs hold):
-// the shortest step wherever the kernels below have none, and for 512 units up to 192 (direction, sequence) pairs, where the chunks of
-// lstm_ptc.cu start to pay (B200, us per step forward / backward, bidirectional: 32 sequences 3.3 / 4.0 here, 4.1 / 4.9 there; 64: 4.7 /
-// 5.9 and 7.2 / 5.5; 128: 9.3 / 10.1 and 9.5 / 10.0; 256: 16.2 / 19.8 and 10.6 / 13.6).  Strict fp32 products (force_ffma) and the other
-// modes stay with the kernels they name.
+// The register-resident cluster kernels serve up to 512 units per direction (what the registers and tensor memory of 16 SMs hold), the
+// shortest step wherever the kernels of lstm_wide.cu are not estimated shorter.  Strict fp32 products (force_ffma) and the other modes stay
+// with the kernels they name.
 bool LstmLayerImpl::want_cluster() const {
-    const LstmShape s = shape();
-    if (force_ffma || recurrence_mode != 1 || !lstm_cluster_supported(s)) return false;
-    return s.D * s.P <= 192 || !lstm_ptc_supported(s);
+    return !force_ffma && recurrence_mode == 1 && lstm_cluster_supported(shape()) && !want_wide();
 }
 
-// The persistent tensor-core kernels serve 512 units per direction.  Modes 5 and 6 force them; the default (mode 1)
-// takes them for fractions too large for the cluster kernels (above).
+// The persistent tensor-core kernels with weights in shared memory only serve 512 units per direction.  Modes 5 and 6 force them; the
+// default (mode 1) takes them where neither the kernels of lstm_wide.cu nor the cluster kernels fit the device.
 bool LstmLayerImpl::want_ptc() const {
     const LstmShape s = shape();
     if (force_ffma || !lstm_ptc_supported(s)) return false;
@@ -374,13 +370,17 @@ bool LstmLayerImpl::want_ptc() const {
     return recurrence_mode == 1 && s.P >= 16;
 }
 
-// The persistent tensor-core kernels of 513 to 1024 units per direction.  Few sequences of 1024 units are left to the FFMA kernels
-// (lstm_persistent.cu), whose step is shorter while one pass of 8 sequences (or one sequence per direction) covers the fraction (B200, us
-// per step forward / backward: one sequence, bidirectional 3.6 / 3.4 there, 4.6 / 5.9 here; unidirectional 1 to 8 sequences 1.8 / 1.7 to
-// 4.9 / 4.8 there, 4.5 / 5.6 here; 2 sequences, bidirectional 9.1 / 9.2 and 4.6 / 5.8).
+// The persistent tensor-core kernels with weights in shared and tensor memory, 257 to 1024 units per direction.
+// Up to 512 units they take the fractions whose sequences need several passes of the cluster kernels (B200, us per step forward / backward,
+// bidirectional, cluster kernels and these: 512 units, 32 sequences 3.8 / 4.0 and 4.5 / 5.9, 64: 5.5 / 5.9 and 4.5 / 6.0, 128: 9.3 / 10.1 and
+// 5.7 / 6.9, 256: 16.2 / 19.8 and 8.0 / 9.3; 300 units, 64: 4.0 / 4.8 and 4.4 / 5.9, 128: 7.6 / 9.5 and 5.8 / 6.9).
+// Few sequences of 1024 units are left to the FFMA kernels (lstm_persistent.cu), whose step is shorter while one pass of 8 sequences (or
+// one sequence per direction) covers the fraction (one sequence, bidirectional 3.6 / 3.4 there, 4.6 / 5.9 here; unidirectional 1 to 8
+// sequences 1.8 / 1.7 to 4.9 / 4.8 there, 4.5 / 5.6 here; 2 sequences, bidirectional 9.1 / 9.2 and 4.6 / 5.8).
 bool LstmLayerImpl::want_wide() const {
     const LstmShape s = shape();
     if (force_ffma || recurrence_mode != 1 || !lstm_wide_supported(s)) return false;
+    if (s.els <= 512) return !lstm_cluster_supported(s) || lstm_wide_step_us(s) < lstm_cluster_step_us(s);
     int JB = 0;
     return !(persistent_geometry(s.els, &JB) && (s.P == 1 || (s.D == 1 && s.P <= 8)));
 }
@@ -388,7 +388,7 @@ bool LstmLayerImpl::want_wide() const {
 int LstmLayerImpl::ensure_wide() {
     if (wide.flags) return B2_OK;
     size_t xb = 0, nf = 0;
-    lstm_wide_sizes(&xb, &nf);
+    lstm_wide_sizes(shape(), &xb, &nf);
     B2_CUDA(cudaMalloc(&wide.xchg, xb));
     B2_CUDA(cudaMalloc(&wide.flags, nf * sizeof(unsigned)));
     B2_CUDA(cudaMemset(wide.xchg, 0, xb));

@@ -1,4 +1,4 @@
-// Persistent tensor-core recurrence for 513 to 1024 units per direction: ONE launch runs all timesteps of a sweep with the
+// Persistent tensor-core recurrence for 257 to 1024 units per direction: ONE launch runs all timesteps of a sweep with the
 // recurrent weights resident on chip, fp16 hi parts in shared memory, lo parts in TENSOR MEMORY.
 //
 // Replaces the reference's per-timestep loop of 4 cublasSgemm + 1 Thrust functor per direction
@@ -16,6 +16,8 @@
 //             8 would not fit 16 times, so the slices of a row tile exchange partial sums through L2.
 // The two sweeps are one kernel: gather an operand slice, multiply, exchange partial sums, run the cells of the 16 units a block
 // finishes, publish what the next step gathers (h, resp. the gate deltas).  Fewer units are padded to 1024 with zero weights.
+// Up to 512 units (padded to 512) a group has 16 blocks and eight groups run side by side, a chunk of sequences each: 16 row tiles with the
+// whole contraction forward (no exchange), 4 row tiles x 4 slices backward; a block finishes 32 units.
 //
 // A step of a chunk of NC sequences (16, 32 or 64).  The operand lies in global memory (L2) as images of 64 contraction positions:
 // 2 NC rows (hi of every sequence, then lo) of 128 bytes, swizzled.  The polling warp watches the step counters of the blocks that
@@ -29,7 +31,8 @@
 // per step forward / backward: one thread issuing all MMAs and a proxy fence before each bulk copy 12.7 / 16.8; several issuers (a
 // tcgen05.mma with run-time descriptors costs its thread 118 cycles) and one fence on the publishing side 10.3 / 14.0; copies issued by 8
 // lanes side by side and the layer's state stored only after the publication 8.4 / 11.8; the counters on lines of their own and
-// partial sums read straight from L2 7.6 / 7.7.  The launch pair per step of lstm_step_tc.cu takes 24.6 / 26.6; 16 sequences: 4.5 / 6.0
+// partial sums read straight from L2 7.6 / 7.7.  512 units, 256 sequences in eight groups: 8.0 / 9.3, of which the cells of 32 units x 64
+// sequences take 2 (lstm_ptc.cu 11.1 / 13.5).  The launch pair per step of lstm_step_tc.cu takes 24.6 / 26.6; 16 sequences: 4.5 / 6.0
 // and 23.0 / 23.8.
 // Numerics as in lstm_ptc.cu: x*S = hi + lo*2^-11, S = 2^14 for h, 2^15 for the deltas, 2^13 <= max|w|*S < 2^14 per block; a chain holds at
 // most 16 main products (tensor-memory accumulation truncates).
@@ -52,7 +55,7 @@ using cluster::cl_logistic;
 using cluster::cl_tanh;
 using cluster::settle;
 
-constexpr int GROUP = 64, UPB = 16, KB = 8;               // blocks of a direction; units a block finishes; images of a slice
+constexpr int KB = 8;                                     // operand images of a slice
 // Step counters: a line of 128 bytes for each slice (fewer readers wait longer for a line that many SMs poll: one line for all slices,
 // polled by 8 warps of a block, cost the backward step of 16 sequences 3 us), in several copies that the readers share; behind them a line
 // for the partial sums of each row tile.
@@ -76,16 +79,19 @@ struct WideArgs {
     int nchunks;             // chunks of NC sequences
 };
 
-template <bool BWD, int NC>
+// E: the units of a direction are padded to E = 1024 or 512
+template <int E, bool BWD, int NC>
 struct Geo {
-    static constexpr int CS = BWD ? 8 : 2, ROWS = 128 / CS;            // slices of a row tile; rows of partial sums a block finishes
-    static constexpr int CL = BWD ? 1 : 2;                             // blocks of a cluster
-    // warps that issue MMAs, each on an accumulator of its own (columns NI x 2 NC <= 256); the other roles follow
-    static constexpr int NI = NC == 64 ? 2 : 4, ACC = 256 / NI;
-    static constexpr int W_DRAIN = W_MMA + NI, W_CELL = W_DRAIN + 4, W_PUB = W_CELL + 8, NTHR = 32 * (W_PUB + 1);
+    static constexpr int GROUP = E * E / 16384, UPB = E / GROUP;       // blocks of a group; units a block finishes
+    static constexpr int CS = BWD ? E / 128 : E / 512, ROWS = 128 / CS;   // slices of a row tile; rows of partial sums a block finishes
+    static constexpr int CL = BWD ? 1 : CS;                            // blocks of a cluster
+    // warps that issue MMAs, each on an accumulator of its own (columns NI x 2 NC <= 256); the other roles follow.  16 sequences side by
+    // side in the cell warps.
+    static constexpr int NI = NC == 64 ? 2 : 4, ACC = 256 / NI, NCW = UPB / 2;
+    static constexpr int W_DRAIN = W_MMA + NI, W_CELL = W_DRAIN + 4, W_PUB = W_CELL + NCW, NTHR = 32 * (W_PUB + 1);
     static constexpr uint32_t IMG = 2 * NC * 128;                      // one operand image
     static constexpr int STAGES = NC == 64 ? 4 : 8;                    // images in flight: a whole slice where shared memory allows it
-    static constexpr int NIMG = BWD ? 64 : 16;                         // images of a whole operand
+    static constexpr int NIMG = BWD ? E / 16 : E / 64;                 // images of a whole operand
     static constexpr uint32_t F_B = A_BYTES, F_Z = F_B + STAGES * IMG; // z: [source][NC / 4][ROWS][4]
     static constexpr uint32_t ZSRC = ROWS * NC * 4, F_END = F_Z + (BWD ? 0 : CS * ZSRC);
     static constexpr size_t smem() { return F_END + 1024; }
@@ -120,9 +126,10 @@ __device__ __forceinline__ void load_l2(const float *p, float (&v)[4]) {
     asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p) : "memory");
 }
 
-template <bool BWD, int NC>
-__global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideArgs a) {
-    typedef Geo<BWD, NC> G;
+template <int E, bool BWD, int NC>
+__global__ void __launch_bounds__(Geo<E, BWD, NC>::NTHR, 1) lstm_wide_kernel(WideArgs a) {
+    typedef Geo<E, BWD, NC> G;
+    constexpr int GROUP = G::GROUP, UPB = G::UPB;
     constexpr int CS = G::CS, ROWS = G::ROWS, STAGES = G::STAGES, NI = G::NI, NTHR = G::NTHR;
     constexpr int W_DRAIN = G::W_DRAIN, W_CELL = G::W_CELL, W_PUB = G::W_PUB, CPT = NC / 16;        // CPT: cells per cell thread
     extern __shared__ unsigned char smem_raw[];
@@ -156,8 +163,8 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
         for (int s = 0; s < STAGES; ++s) { mbar_init(b_full(s), 1); mbar_init(b_free(s), 1); }
         mbar_init(acc_full, NI); mbar_init(acc_free, 4);
         mbar_init(z_full, BWD ? 1 : 5);       // forward: 4 drain warps and the arrival that announces the peer's bytes; backward: poll warp
-        mbar_init(z_free, 8 * G::CL);         // every cell warp of every block of the cluster
-        mbar_init(rel_full, 8); mbar_init(rel_free, 1);
+        mbar_init(z_free, G::NCW * G::CL);         // every cell warp of every block of the cluster
+        mbar_init(rel_full, G::NCW); mbar_init(rel_free, 1);
         mbar_init(part_full, 4);
         for (int h = 0; h < NI; ++h) mbar_init(quit + 8u * (uint32_t)h, 1);
         give_up_s = 0; never_s = 0;
@@ -165,7 +172,7 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
     }
     if (warp == 0) tmem_alloc(smem_u32(&tmem_base_s), 512);
     tc_fence_before();
-    if constexpr (BWD) __syncthreads(); else cluster_sync_all();     // a peer's shared memory and barriers may be touched only once the peer runs
+    if constexpr (G::CL == 1) __syncthreads(); else cluster_sync_all();     // a peer's shared memory and barriers may be touched only once the peer runs
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;      // columns 0-255: accumulators [half][main NC | cross NC], 256-511: lo parts of the weights
 
@@ -241,7 +248,6 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
 
         if (warp == W_POLL) {
             // ---------------- watch the writers of this slice's images, fetch image by image ----------------
-            constexpr int PER = NW / KB;                         // writers of an image
             const unsigned *line = flags + (q * COPIES + r % COPIES) * LINE + lane;
             unsigned late = 0u;                                  // images of an unfinished step that are on their way
             for (int s = 1; s < Tc; ++s) {
@@ -250,7 +256,8 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
                 const unsigned char *src = img + ((size_t)((ev + (unsigned)(s - 1)) & 1u) * G::NIMG + (size_t)(KB * q)) * G::IMG;
                 // lane = place of an image in the order of fetching: the parts of the slice in turn, an issuing warp takes each
                 const int kb = (lane & 7) / NI + KB / NI * (lane % NI), nb = n_b + (lane & 7), st = nb % STAGES;
-                const unsigned need = (PER == 1 ? 1u : 15u) << (PER * kb);
+                // writers of this image: 64 units of h, or the gate deltas of 16 units
+                const unsigned need = BWD ? 1u << (16 * kb / UPB) : ((1u << (64 / UPB)) - 1u) << (64 / UPB * kb);
                 constexpr unsigned ALL = (1u << KB) - 1u;
                 unsigned ready = 0u, sent = 0u;
                 bool ok = true;
@@ -317,11 +324,11 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
         } else if (warp < W_CELL) {
             // ---------------- drain tensor memory: every row to the block that finishes its unit ----------------
             const int row = 32 * (warp & 3) + lane;
-            const int to = BWD ? row / ROWS : (row & 31) >> 4;                            // rank of that block
-            const int rl = BWD ? row % ROWS : (row >> 5) * UPB + (row & 15);              // row among its ROWS
+            const int to = BWD ? row / ROWS : (row & 31) / UPB;                           // rank of that block
+            const int rl = BWD ? row % ROWS : (row >> 5) * UPB + row % UPB;              // row among its ROWS
             const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
             const uint32_t zl = G::F_Z + (uint32_t)q * G::ZSRC + (uint32_t)rl * 16u;
-            const uint32_t zr = BWD ? 0u : map_to_rank(sbase + zl, (uint32_t)to), rbar = BWD ? 0u : map_to_rank(z_full, (uint32_t)to);
+            const uint32_t zr = G::CL == 1 ? 0u : map_to_rank(sbase + zl, (uint32_t)to), rbar = G::CL == 1 ? 0u : map_to_rank(z_full, (uint32_t)to);
             for (int s = 1; s < Tc; ++s, ++n_d) {
                 if (__any_sync(0xffffffffu, give_up_s)) break;
                 const uint32_t ph = (uint32_t)n_d & 1u;
@@ -360,7 +367,7 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
                         const uint32_t o = (uint32_t)((col >> 2) + g4) * (ROWS * 16u);
                         if constexpr (BWD)
                             *reinterpret_cast<float4 *>(zg + o) = make_float4(v[4 * g4], v[4 * g4 + 1], v[4 * g4 + 2], v[4 * g4 + 3]);
-                        else if (to == q)
+                        else if (G::CL == 1 || to == q)
                             *reinterpret_cast<float4 *>(gbase + zl + o) = make_float4(v[4 * g4], v[4 * g4 + 1], v[4 * g4 + 2], v[4 * g4 + 3]);
                         else
                             st_async_v4(zr + o, __float_as_uint(v[4 * g4]), __float_as_uint(v[4 * g4 + 1]), __float_as_uint(v[4 * g4 + 2]),
@@ -395,8 +402,8 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
                 if (!ok) { give_up_s = 1; atomicCAS(a.status, 0, (int)B2_ERR_STEP_TIMEOUT); break; }
             }
         } else {
-            // ---------------- cells: thread = unit (of 16) of CPT sequences ----------------
-            const int ct = tid - 32 * W_CELL, ul = ct & 15, n0 = ct >> 4;
+            // ---------------- cells: thread = unit (of UPB) of CPT sequences ----------------
+            const int ct = tid - 32 * W_CELL, ul = ct % UPB, n0 = ct / UPB;
             const int j = (BWD ? 128 : 32) * r + UPB * q + ul;                 // unit inside the direction
             const bool unit = j < els;
             auto seq = [&](int i) { return BWD ? n0 * CPT + i : n0 + 16 * i; };     // sequence of this thread's i-th cell
@@ -495,7 +502,11 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
                             }
                         }
                         __syncwarp();
-                        if (lane < CS) mbar_arrive_cluster_relaxed(map_to_rank(z_free, (uint32_t)lane));
+                        if constexpr (G::CL == 1) {
+                            if (lane == 0) mbar_arrive(z_free);
+                        } else if (lane < CS) {
+                            mbar_arrive_cluster_relaxed(map_to_rank(z_free, (uint32_t)lane));
+                        }
                     }
                 }
                 unsigned char *dst = img + (size_t)((ev + (unsigned)s) & 1u) * G::NIMG * G::IMG;
@@ -538,7 +549,7 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
                         if (!last) {
                             // contraction position 4 * unit + gate: this thread's four gates are 8 bytes of each part
                             const unsigned v0 = split_pair(dd[0], S_D), v1 = split_pair(dd[1], S_D), v2 = split_pair(dd[2], S_D), v3 = split_pair(dd[3], S_D);
-                            unsigned char *c8 = dst + (size_t)(8 * r + q) * G::IMG + (size_t)n * 128 + (size_t)(((ul >> 1) ^ (n & 7)) * 16 + 8 * (ul & 1));
+                            unsigned char *c8 = dst + (size_t)(j >> 4) * G::IMG + (size_t)n * 128 + (size_t)((((ul & 15) >> 1) ^ (n & 7)) * 16 + 8 * (ul & 1));
                             *reinterpret_cast<uint2 *>(c8) = make_uint2((v0 & 0xffffu) | (v1 << 16), (v2 & 0xffffu) | (v3 << 16));
                             *reinterpret_cast<uint2 *>(c8 + NC * 128) = make_uint2((v0 >> 16) | (v1 & 0xffff0000u), (v2 >> 16) | (v3 & 0xffff0000u));
                         }
@@ -592,67 +603,69 @@ __global__ void __launch_bounds__(Geo<BWD, NC>::NTHR, 1) lstm_wide_kernel(WideAr
     tc_fence_before();
     __syncthreads();
     if (give_up_s && tid == 0) atomicCAS(a.status, 0, (int)B2_ERR_STEP_TIMEOUT);
-    if constexpr (!BWD) cluster_sync_all();      // nobody leaves while a peer may still write into its shared memory
+    if constexpr (G::CL > 1) cluster_sync_all();      // nobody leaves while a peer may still write into its shared memory
     tc_fence_after();
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 typedef void (*WideKernel)(WideArgs);
 constexpr int NVARIANTS = 3, CHUNK[NVARIANTS] = {16, 32, 64};
-WideKernel kernel_of(bool backward, int v) {
-    static const WideKernel k[2][NVARIANTS] = {{lstm_wide_kernel<false, 16>, lstm_wide_kernel<false, 32>, lstm_wide_kernel<false, 64>},
-                                               {lstm_wide_kernel<true, 16>, lstm_wide_kernel<true, 32>, lstm_wide_kernel<true, 64>}};
-    return k[backward][v];
+struct Variant { WideKernel kern; int group, cluster, threads; size_t smem, xchg; };
+template <int E, bool BWD, int NC>
+constexpr Variant variant_of() {
+    typedef Geo<E, BWD, NC> G;
+    return Variant{lstm_wide_kernel<E, BWD, NC>, G::GROUP, G::CL, G::NTHR, G::smem(), G::GROUP_BYTES};
 }
-size_t smem_of(bool backward, int v) {
-    static const size_t k[2][NVARIANTS] = {{Geo<false, 16>::smem(), Geo<false, 32>::smem(), Geo<false, 64>::smem()},
-                                           {Geo<true, 16>::smem(), Geo<true, 32>::smem(), Geo<true, 64>::smem()}};
-    return k[backward][v];
-}
-void launch_config(bool backward, int v, int blocks, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute (*attr)[2]) {
+#define CHUNKS(E, BWD) {variant_of<E, BWD, 16>(), variant_of<E, BWD, 32>(), variant_of<E, BWD, 64>()}
+const Variant VARIANTS[2][2][NVARIANTS] = {{CHUNKS(512, false), CHUNKS(512, true)}, {CHUNKS(1024, false), CHUNKS(1024, true)}};   // [wide][backward]
+
+void launch_config(const Variant &v, int groups, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute (*attr)[2]) {
     (*attr)[0].id = cudaLaunchAttributeCooperative;
     (*attr)[0].val.cooperative = 1;
     (*attr)[1].id = cudaLaunchAttributeClusterDimension;
-    (*attr)[1].val.clusterDim.x = 2; (*attr)[1].val.clusterDim.y = 1; (*attr)[1].val.clusterDim.z = 1;
+    (*attr)[1].val.clusterDim.x = v.cluster; (*attr)[1].val.clusterDim.y = 1; (*attr)[1].val.clusterDim.z = 1;
     *cfg = cudaLaunchConfig_t{};
-    cfg->gridDim = dim3(blocks);
-    cfg->blockDim = dim3(v == 2 ? Geo<false, 64>::NTHR : Geo<false, 32>::NTHR);
-    cfg->dynamicSmemBytes = smem_of(backward, v);
+    cfg->gridDim = dim3(groups * v.group);
+    cfg->blockDim = dim3(v.threads);
+    cfg->dynamicSmemBytes = v.smem;
     cfg->stream = st;
     cfg->attrs = *attr;
-    cfg->numAttrs = backward ? 1 : 2;
+    cfg->numAttrs = v.cluster > 1 ? 2 : 1;
 }
-// groups of 64 blocks that the current device holds at once
-int resident_groups() {
+// groups that the current device holds at once, at most those the exchange buffers are made for
+constexpr int MAX_GROUPS[2] = {8, 2};
+int resident_groups(bool wide) {
     static std::mutex mu;
-    static short known[MAX_DEVICES];      // 0 = not asked yet, else groups + 1
+    static short known[MAX_DEVICES][2];      // 0 = not asked yet, else groups + 1
     const int dev = current_device();
     if (dev < 0) return 0;
     std::lock_guard<std::mutex> lk(mu);
-    if (!known[dev]) {
-        int groups = sm_count() / GROUP;
-        for (int v = 0; v < NVARIANTS; ++v) {
+    if (!known[dev][wide]) {
+        int groups = std::min(MAX_GROUPS[wide], sm_count() / VARIANTS[wide][0][0].group);
+        for (int i = 0; wide && i < NVARIANTS; ++i) {
+            const Variant &v = VARIANTS[wide][0][i];
             int n = 0;
             cudaLaunchConfig_t cfg;
             cudaLaunchAttribute attr[2];
-            launch_config(false, v, GROUP, nullptr, &cfg, &attr);
-            if (cudaFuncSetAttribute((const void *)kernel_of(false, v), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(false, v)) != cudaSuccess ||
-                cudaOccupancyMaxActiveClusters(&n, kernel_of(false, v), &cfg) != cudaSuccess) {
+            launch_config(v, 1, nullptr, &cfg, &attr);
+            if (cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, v.kern, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 n = 0;
             }
-            groups = std::min(groups, 2 * n / GROUP);
+            groups = std::min(groups, v.cluster * n / v.group);
         }
-        known[dev] = (short)(groups + 1);
+        known[dev][wide] = (short)(groups + 1);
     }
-    return known[dev] - 1;
+    return known[dev][wide] - 1;
 }
-// The smallest chunk that leaves every group one work item (us per step on a B200, forward / backward: chunks of 16 4.5 / 6.0, of 32
-// 5.4 / 7.0, of 64 7.6 / 7.7), else chunks of 64.
-struct Plan { int v, nchunks, groups; };
+// The smallest chunk that leaves every group one work item (us per step on a B200, 1024 units, forward / backward: chunks of 16 4.5 / 6.0, of
+// 32 5.4 / 7.0, of 64 7.6 / 7.7), else chunks of 64.
+struct Plan { bool wide; int v, nchunks, groups; };
 Plan make_plan(const LstmShape &s) {
-    const int room = std::min(2, resident_groups()), share = room > s.D ? (s.P + 1) / 2 : s.P;
     Plan p;
+    p.wide = s.els > 512;
+    const int room = resident_groups(p.wide), per_dir = room > s.D ? room / s.D : 1, share = (s.P + per_dir - 1) / per_dir;
     p.v = share <= 16 ? 0 : (share <= 32 ? 1 : 2);
     p.nchunks = (s.P + CHUNK[p.v] - 1) / CHUNK[p.v];
     p.groups = std::min(room, s.D * p.nchunks);
@@ -661,28 +674,38 @@ Plan make_plan(const LstmShape &s) {
 
 }  // namespace
 
-bool lstm_wide_supported(const LstmShape &s) { return s.els > 512 && s.els <= 1024 && s.P >= 1 && resident_groups() >= 1; }
+// measured on a B200: a step of the forward sweep and one of the backward sweep, for each work item of a group
+double lstm_wide_step_us(const LstmShape &s) {
+    static const double us[2][NVARIANTS] = {{10.5, 12.5, 17.3}, {10.5, 12.4, 15.3}};
+    const Plan p = make_plan(s);
+    return us[p.wide][p.v] * ((s.D * p.nchunks + p.groups - 1) / p.groups);
+}
 
-void lstm_wide_sizes(size_t *exchange_bytes, size_t *flag_words) {
-    *exchange_bytes = 2 * std::max(Geo<false, 64>::GROUP_BYTES, Geo<true, 64>::GROUP_BYTES);
-    *flag_words = 2 * GROUP_FLAGS;
+bool lstm_wide_supported(const LstmShape &s) { return s.els > 256 && s.els <= 1024 && s.P >= 1 && resident_groups(s.els > 512) >= 1; }
+
+void lstm_wide_sizes(const LstmShape &s, size_t *exchange_bytes, size_t *flag_words) {
+    const bool wide = s.els > 512;
+    *exchange_bytes = 0;
+    for (int b = 0; b < 2; ++b)
+        for (int i = 0; i < NVARIANTS; ++i) *exchange_bytes = std::max(*exchange_bytes, MAX_GROUPS[wide] * VARIANTS[wide][b][i].xchg);
+    *flag_words = (size_t)MAX_GROUPS[wide] * GROUP_FLAGS;
 }
 
 int lstm_wide_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, const WideBuffers &wb, const float *w, float *y, const float *dy,
                     int *status, unsigned *tag_next, cudaStream_t st) {
     if (!lstm_wide_supported(s)) return 1;
     const Plan pl = make_plan(s);
-    const int v = pl.v;
+    const Variant &v = VARIANTS[pl.wide][backward][pl.v];
     WideArgs a;
     a.sh = s; a.bf = b; a.w = w; a.y = y; a.dy = dy;
     a.img = wb.xchg; a.flags = wb.flags; a.status = status;
     a.tag_base = *tag_next;
     a.nchunks = pl.nchunks;
-    B2_TRY(set_max_dynamic_smem((const void *)kernel_of(backward, v), (int)smem_of(backward, v)));
+    B2_TRY(set_max_dynamic_smem((const void *)v.kern, (int)v.smem));
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    launch_config(backward, v, pl.groups * GROUP, st, &cfg, &attr);
-    B2_CUDA(cudaLaunchKernelEx(&cfg, kernel_of(backward, v), a));
+    launch_config(v, pl.groups, st, &cfg, &attr);
+    B2_CUDA(cudaLaunchKernelEx(&cfg, v.kern, a));
     count_launch();
     *tag_next += (unsigned)(s.D * a.nchunks) * ((unsigned)s.T + 1u);
     return B2_OK;

@@ -559,9 +559,10 @@ def test_cluster_recurrence(els, bi, P, T):
 
 
 @pytest.mark.parametrize("els,bi,P,T", [(513, 1, 2, 5), (1024, 0, 9, 6), (1024, 1, 16, 4), (600, 1, 17, 5), (1023, 1, 33, 4), (640, 0, 33, 7),
-                                        (1024, 1, 65, 4), (776, 0, 130, 3), (1024, 1, 2, 1), (800, 1, 1, 40)])
+                                        (1024, 1, 65, 4), (776, 0, 130, 3), (1024, 1, 2, 1), (800, 1, 1, 40), (512, 1, 64, 7), (500, 1, 128, 5),
+                                        (384, 0, 500, 4), (257, 1, 250, 4), (512, 1, 520, 3)])
 def test_wide_recurrence(els, bi, P, T):
-    """The persistent kernels of 513 to 1024 units per direction: every chunk size, several chunks of a group, chunks whose sequences all
+    """The persistent kernels with weights in shared and tensor memory: every chunk size, several chunks of a group, chunks whose sequences all
     end early, unit counts that pad a block's units or whole blocks, one step."""
     from b2lstm import workloads
     ls = els * (2 if bi else 1)
