@@ -161,8 +161,6 @@ struct LstmBuffers {
     float *cerr;        // [2][P][ls]:  cell-state errors of the two most recent steps (stepwise kernels)
     float *wrecT;       // [D][els][4][els]: recurrent weights, source unit major (forward sweep)
     const char *pat;    // [T*P]
-    const int *real = nullptr;   // the real frames of the fraction, n_real of them (NULL: take all frames)
-    int n_real = 0;
 };
 // one launch per timestep, both directions in the same launch
 int lstm_forward_stepwise(const LstmShape &s, const LstmBuffers &b, const float *w, float *y, cudaStream_t st);
@@ -170,8 +168,8 @@ int lstm_backward_stepwise(const LstmShape &s, const LstmBuffers &b, const float
                            cudaStream_t st);
 // transpose the recurrent block of the weight vector into LstmBuffers::wrecT
 int lstm_prepare_wrecT(const LstmShape &s, const float *w, float *wrecT, cudaStream_t st);
-// bias and peephole gradients (the vector part of the weight update), written into dw
-int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, float *dw, float *ws, size_t ws_floats,
+// bias and peephole gradients (the vector part of the weight update), written into dw; real: the frames to sum over (NULL: all)
+int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *real, int n_real, float *dw, float *ws, size_t ws_floats,
                       cudaStream_t st);
 
 // tensor-core recurrence for large batches (lstm_step_tc.cu): one batched tcgen05 GEMM + one gate

@@ -116,7 +116,7 @@ int LstmLayerImpl::load_sequences(int cur_max, int cur_min, const char *pat) {
             return B2_ERR_BAD_ARG;
         }
     }
-    T = cur_max; Tmin = cur_min; bufs.pat = pat; bufs.real = nullptr; bufs.n_real = 0;
+    T = cur_max; Tmin = cur_min; bufs.pat = pat; real = nullptr; n_real = 0;
     forward_done = false;
     return B2_OK;
 }
@@ -127,7 +127,7 @@ int LstmLayerImpl::load_sequences(int cur_max, int cur_min, const char *pat) {
 void LstmLayerImpl::set_real_frames(const int *map, int n) {
     const long frames = (long)T * desc.parallel_sequences;
     if (!map || n < 1 || (long)n > frames - frames / 16) return;
-    bufs.real = map; bufs.n_real = n;
+    real = map; n_real = n;
 }
 
 int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_t st) {
@@ -139,14 +139,14 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
     // LstmLayer.cu:1756-1775): acts(4ls x N) = W_in^T X, W_in viewed as ONE pls x 4ls matrix
     {
         Phase ph(*this, "lstm_proj_gemm");
-        if (bufs.real && !force_ffma && scratch && gemm_wants_tc(pls, 1, 1, pls, 4 * ls, bufs.n_real, pls)) {
-            B2_TRY(scratch->reserve(split_floats(4 * ls, pls) + split_floats(bufs.n_real, pls)));
+        if (real && !force_ffma && scratch && gemm_wants_tc(pls, 1, 1, pls, 4 * ls, n_real, pls)) {
+            B2_TRY(scratch->reserve(split_floats(4 * ls, pls) + split_floats(n_real, pls)));
             scratch->used = 0;
             SplitOperand sW{}, sX{};
-            SplitJob jobs[2] = {{w, pls, 4 * ls, pls, true, 0.0f, &sW}, {x, pls, bufs.n_real, pls, true, x_bound, &sX}};
-            jobs[1].map = bufs.real;
+            SplitJob jobs[2] = {{w, pls, 4 * ls, pls, true, 0.0f, &sW}, {x, pls, n_real, pls, true, x_bound, &sX}};
+            jobs[1].map = real;
             B2_TRY(split_operands(*scratch, jobs, 2, st));
-            B2_TRY(gemm_tc(bufs.acts, 4 * ls, sW, sX, 4 * ls, bufs.n_real, pls, false, ws, ws_floats, status_dev, st, bufs.real));
+            B2_TRY(gemm_tc(bufs.acts, 4 * ls, sW, sX, 4 * ls, n_real, pls, false, ws, ws_floats, status_dev, st, real));
         } else {
             B2_TRY(gemm_auto(bufs.acts, 4 * ls, w, pls, 1, x, 1, pls, 4 * ls, N, pls, false, force_ffma, scratch, ws, ws_floats, status_dev,
                              st, x_bound));
@@ -226,8 +226,7 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
         if (rc == 1) { rc = lstm_backward_stepwise(s, bufs, w, dy, st); bwd_path = 0; }
         B2_TRY(rc);
     }
-    const int *real = bufs.real;
-    const int NR = real ? bufs.n_real : N;      // frames the products run over
+    const int NR = real ? n_real : N;      // frames the products run over
     const bool tc = !force_ffma && scratch && gemm_wants_tc(1, pls, 4 * ls, 1, pls, 4 * ls, NR);
     // contraction length of the recurrent weight gradients: the list of real frames pairs every delta with the h of the step before (its
     // operand is gathered with a shift), the frames in their order pair all but one timestep
@@ -330,7 +329,7 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
             }
     }
     Phase ph(*this, "lstm_vector_grads");
-    B2_TRY(lstm_vector_grads(s, bufs, dw, ws, ws_floats, st));
+    B2_TRY(lstm_vector_grads(s, bufs, real, n_real, dw, ws, ws_floats, st));
     return B2_OK;
 }
 

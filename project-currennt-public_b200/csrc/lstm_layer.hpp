@@ -15,6 +15,8 @@ struct LstmLayerImpl {
     bool check_padding = false;   // load_sequences verifies that padding frames trail their sequences
     int *pad_dev = nullptr;       // result word of that check
     LstmBuffers bufs{};
+    const int *real = nullptr;    // the real frames of the fraction, n_real of them (NULL: the products take all frames)
+    int n_real = 0;
     float *ws = nullptr;       // scratch: split-K partials, vector-gradient partials
     size_t ws_floats = 0;
     size_t state_bytes = 0;
