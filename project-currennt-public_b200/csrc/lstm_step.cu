@@ -289,7 +289,9 @@ int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *real,
                       cudaStream_t st) {
     const long N = real ? n_real : (long)s.T * s.P;
     // chunks of frames: enough blocks to fill the device several times over, bounded by the scratch
-    int fpc = 64;
+    // (800 frames x 128 units, 64 frames a chunk: 13 blocks, each a chain of 16 rounds of loads)
+    long fit = N * ((s.ls + 127) / 128) / (4 * sm_count());
+    int fpc = fit < 8 ? 8 : (fit > 64 ? 64 : (int)fit);
     const long max_chunks = (long)(ws_floats / ((size_t)7 * s.ls));
     if (max_chunks < 1) {
         set_error("lstm_vector_grads: scratch too small");
