@@ -553,9 +553,16 @@ __global__ void __launch_bounds__(256) absmax_batch_kernel(const __grid_constant
             m = max(m, max(max(finite_bits(x.x), finite_bits(x.y)), max(finite_bits(x.z), finite_bits(x.w))));
         }
     } else if (w.s_outer == w.inner && !w.map) {
-        const size_t total = (size_t)w.outer * w.inner;
+        // rows without gaps: one array, whatever their length
+        const size_t total = (size_t)w.outer * w.inner, head = min(total, (size_t)((16 - ((size_t)w.src & 15)) & 15) / 4), n4 = (total - head) / 4;
+        const float4 *p4 = (const float4 *)(w.src + head);
 #pragma unroll 4
-        for (size_t i = i0; i < total; i += stride) m = max(m, finite_bits(__ldg(w.src + i)));
+        for (size_t i = i0; i < n4; i += stride) {
+            const float4 x = __ldg(p4 + i);
+            m = max(m, max(max(finite_bits(x.x), finite_bits(x.y)), max(finite_bits(x.z), finite_bits(x.w))));
+        }
+        if (i0 < head) m = max(m, finite_bits(__ldg(w.src + i0)));
+        if (i0 < total - head - 4 * n4) m = max(m, finite_bits(__ldg(w.src + head + 4 * n4 + i0)));
     } else {
         // a warp per row
         for (int r = block * 8 + (int)(threadIdx.x >> 5); r < w.outer; r += w.parts * 8)
