@@ -141,6 +141,9 @@ int sgd_update_opt(float *w, float *g, float *delta, float *stats, size_t n, flo
                    const float *frac_len_dev, float beta1_accum, float beta2_accum, cudaStream_t st);
 // pattern types and list of the real frames of a fraction from its sequence lengths (lens: P lengths, P running sums, on the device)
 int fraction_maps(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st);
+// the same with the lengths in host memory, up to MAX_ARG_LENS sequences
+constexpr int MAX_ARG_LENS = 256;
+int fraction_maps_args(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st);
 // zeroes the rows of m(frames x cols) that belong to padding frames
 int zero_padding_rows(float *m, int cols, const char *pat, int frames, cudaStream_t st);
 int fill_value(float *p, size_t n, float v, cudaStream_t st);

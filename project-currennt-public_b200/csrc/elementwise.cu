@@ -272,6 +272,15 @@ int accumulate(float *acc, const float *g, size_t n, bool first, cudaStream_t st
 // Pattern types of a fraction (1 first, 2 inner, 3 last frame of a sequence, 0 padding) and the list of its real frames, sequence by
 // sequence; one thread per frame.  lens[0..P) are the lengths, lens[P..2P) their running sums.
 namespace {
+struct FractionLens { int len[MAX_ARG_LENS], sum[MAX_ARG_LENS]; };
+// few sequences: the lengths come as kernel arguments, which saves the copy
+__global__ void fraction_args_kernel(const __grid_constant__ FractionLens l, int P, int frames, char *__restrict__ pat, int *__restrict__ map) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= frames) return;
+    const int t = f / P, p = f - t * P, len = l.len[p];
+    pat[f] = t >= len ? PAT_NONE : (t == 0 ? 1 : (t == len - 1 ? 3 : 2));
+    if (t < len) map[l.sum[p] + t] = f;
+}
 __global__ void fraction_kernel(const int *__restrict__ lens, int P, int frames, char *__restrict__ pat, int *__restrict__ map) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= frames) return;
@@ -287,6 +296,14 @@ __global__ void zero_padding_kernel(float *__restrict__ m, int cols, const char 
 }  // namespace
 int fraction_maps(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st) {
     fraction_kernel<<<(frames + 255) / 256, 256, 0, st>>>(lens, P, frames, pat, map);
+    count_launch();
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+int fraction_maps_args(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st) {
+    FractionLens l;
+    for (int p = 0; p < P; ++p) { l.len[p] = lens[p]; l.sum[p] = lens[P + p]; }
+    fraction_args_kernel<<<(frames + 255) / 256, 256, 0, st>>>(l, P, frames, pat, map);
     count_launch();
     B2_CUDA(cudaGetLastError());
     return B2_OK;

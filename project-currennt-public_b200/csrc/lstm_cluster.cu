@@ -714,7 +714,7 @@ double step_cycles(const Variant &v, int KP, int nt, double share, bool backward
 }
 
 struct Plan { int vi, nt, items, clusters; double cycles; };
-Plan make_plan(const LstmShape &s, bool backward) {
+Plan search_plan(const LstmShape &s, bool backward) {
     Plan best{-1, 0, 0, 0, 0.0};
     double best_t = 0.0;
     const int tiles = (s.P + 7) / 8;
@@ -735,6 +735,24 @@ Plan make_plan(const LstmShape &s, bool backward) {
         }
     }
     return best;
+}
+
+// a layer asks for its plan several times a pass (the search takes 5 us of host time): every thread keeps those of the last shapes it met
+Plan make_plan(const LstmShape &s, bool backward) {
+    struct Memo { int dev, els, D, P; Plan plan; };
+    constexpr int N = 16;
+    static thread_local Memo memo[2][N];
+    static thread_local int used[2], next[2];
+    const int dev = current_device();
+    for (int i = 0; i < used[backward]; ++i) {
+        const Memo &m = memo[backward][i];
+        if (m.dev == dev && m.els == s.els && m.D == s.D && m.P == s.P) return m.plan;
+    }
+    const Memo m{dev, s.els, s.D, s.P, search_plan(s, backward)};
+    memo[backward][next[backward]] = m;
+    next[backward] = (next[backward] + 1) % N;
+    if (used[backward] < N) ++used[backward];
+    return m.plan;
 }
 
 }  // namespace

@@ -423,16 +423,21 @@ int NeuralNetwork::stageFraction(int b, int T, int nSeq, const int *lens, const 
     // pattern types as DataSet::_makeFractionTask writes them (data_sets/DataSet.cpp:853-861)
     size_t frames = (size_t)mx * P;
     int *lh = lenPinned[b];
+    const bool args = P <= MAX_ARG_LENS;
     // the pinned staging is rewritten by the host: the previous copy out of it must have run
-    B2_CUDA(cudaEventSynchronize(patCopied[b]));
+    if (!args) B2_CUDA(cudaEventSynchronize(patCopied[b]));
     for (int p = 0, sum = 0; p < P; ++p) {
         lh[p] = p < nSeq ? lens[p] : 0;
         lh[P + p] = sum;
         sum += lh[p];
     }
-    B2_CUDA(cudaMemcpyAsync(lenBuf[b], lh, (size_t)2 * P * sizeof(int), cudaMemcpyHostToDevice, st));
-    B2_CUDA(cudaEventRecord(patCopied[b], st));
-    B2_TRY(fraction_maps(lenBuf[b], P, (int)frames, patBuf[b], mapBuf[b], st));
+    if (args) {
+        B2_TRY(fraction_maps_args(lh, P, (int)frames, patBuf[b], mapBuf[b], st));
+    } else {
+        B2_CUDA(cudaMemcpyAsync(lenBuf[b], lh, (size_t)2 * P * sizeof(int), cudaMemcpyHostToDevice, st));
+        B2_CUDA(cudaEventRecord(patCopied[b], st));
+        B2_TRY(fraction_maps(lenBuf[b], P, (int)frames, patBuf[b], mapBuf[b], st));
+    }
     cudaMemcpyKind kind = onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     B2_CUDA(cudaMemcpyAsync(inBuf[b], in, frames * layers.front()->size() * sizeof(float), kind, st));
     B2_CUDA(cudaMemcpyAsync(tgBuf[b], tg, frames * layers.back()->size() * sizeof(float), kind, st));
