@@ -346,8 +346,10 @@ int NeuralNetwork::create(const char *networkJson, int P_, int maxT_, unsigned s
         B2_CUDA(cudaMalloc(&tgBuf[b], frames * layers.back()->size() * sizeof(float)));
         B2_CUDA(cudaMalloc(&patBuf[b], frames));
         B2_CUDA(cudaMalloc(&mapBuf[b], frames * sizeof(int)));
-        B2_CUDA(cudaMalloc(&lenBuf[b], (size_t)2 * P * sizeof(int)));
-        B2_CUDA(cudaMallocHost(&lenPinned[b], (size_t)2 * P * sizeof(int)));
+        if (P > MAX_ARG_LENS) {
+            B2_CUDA(cudaMalloc(&lenBuf[b], (size_t)2 * P * sizeof(int)));
+            B2_CUDA(cudaMallocHost(&lenPinned[b], (size_t)2 * P * sizeof(int)));
+        }
         B2_CUDA(cudaEventCreateWithFlags(&prefetchDone[b], cudaEventDisableTiming));
         B2_CUDA(cudaEventCreateWithFlags(&bufFree[b], cudaEventDisableTiming));
         B2_CUDA(cudaEventCreateWithFlags(&patCopied[b], cudaEventDisableTiming));
@@ -422,8 +424,8 @@ int NeuralNetwork::stageFraction(int b, int T, int nSeq, const int *lens, const 
     }
     // pattern types as DataSet::_makeFractionTask writes them (data_sets/DataSet.cpp:853-861)
     size_t frames = (size_t)mx * P;
-    int *lh = lenPinned[b];
     const bool args = P <= MAX_ARG_LENS;
+    int la[2 * MAX_ARG_LENS], *lh = args ? la : lenPinned[b];
     // the pinned staging is rewritten by the host: the previous copy out of it must have run
     if (!args) B2_CUDA(cudaEventSynchronize(patCopied[b]));
     for (int p = 0, sum = 0; p < P; ++p) {

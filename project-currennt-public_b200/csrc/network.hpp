@@ -190,7 +190,7 @@ public:
     char *patBuf[2] = {nullptr, nullptr};
     int *mapBuf[2] = {nullptr, nullptr};       // the real frames of the fraction
     int *lenBuf[2] = {nullptr, nullptr};       // sequence lengths and their running sums
-    int *lenPinned[2] = {nullptr, nullptr};    // ... pinned host staging
+    int *lenPinned[2] = {nullptr, nullptr};    // ... pinned host staging (both only for more than MAX_ARG_LENS sequences)
     Fraction fracBuf[2];
     int cur = 0;
     bool prefetchPending = false;
