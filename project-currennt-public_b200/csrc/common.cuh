@@ -127,7 +127,7 @@ int ff_bias_act(float *y, const float *b, float bias, int ls, size_t n, int act,
 int ff_delta(float *err, const float *y, size_t n, int act, cudaStream_t st);
 // out[u] = scale * sum_f m[f*ld + u], u < cols, f < rows; deterministic two-stage reduction
 int column_sums(float *out, const float *m, long ld, int cols, long rows, float scale, float *ws, size_t ws_floats,
-                cudaStream_t st);
+                cudaStream_t st, const int *map = nullptr);   // map: the rows to sum (NULL: the first `rows`)
 // SSE: err_partial -> *loss_dev (double) = 0.5*sum (t-y)^2 over non-padding frames
 int sse_loss(double *loss_dev, const float *y, const float *tgt, const char *pat, int ls, size_t frames, double *ws,
              cudaStream_t st);

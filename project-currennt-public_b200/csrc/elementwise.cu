@@ -58,13 +58,13 @@ __global__ void ff_delta_kernel(float *__restrict__ err, const float *__restrict
 }
 
 __global__ void column_sums_partial_kernel(float *__restrict__ ws, const float *__restrict__ m, long ld, int cols,
-                                           long rows, int rows_per_chunk) {
+                                           long rows, int rows_per_chunk, const int *__restrict__ map) {
     int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= cols) return;
     long r0 = (long)blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
     float s = 0.0f;
 #pragma unroll 8
-    for (long r = r0; r < r1; ++r) s += m[(size_t)r * ld + u];
+    for (long r = r0; r < r1; ++r) s += m[(size_t)(map ? __ldg(map + r) : r) * ld + u];
     ws[(size_t)blockIdx.y * cols + u] = s;
 }
 // 32 columns x 8 chunk phases per block: phase y adds chunks y, y+8, ...; the 8 sums are added in fixed order
@@ -204,9 +204,10 @@ int ff_delta(float *err, const float *y, size_t n, int act, cudaStream_t st) {
 }
 
 int column_sums(float *out, const float *m, long ld, int cols, long rows, float scale, float *ws, size_t ws_floats,
-                cudaStream_t st) {
+                cudaStream_t st, const int *map) {
     // rows (frames) per partial sum: enough blocks to fill the device several times, bounded by the scratch
-    int rpc = 64;
+    const long fit = rows * ((cols + 127) / 128) / (4 * sm_count());
+    int rpc = fit < 8 ? 8 : (fit > 64 ? 64 : (int)fit);
     const long max_chunks = cols > 0 ? (long)(ws_floats / (size_t)cols) : 0;
     if (max_chunks < 1) {
         set_error("column_sums: scratch too small");
@@ -216,7 +217,7 @@ int column_sums(float *out, const float *m, long ld, int cols, long rows, float 
     int chunks = (int)((rows + rpc - 1) / rpc);
     if (chunks < 1) chunks = 1;
     dim3 grid((cols + 127) / 128, chunks);
-    column_sums_partial_kernel<<<grid, 128, 0, st>>>(ws, m, ld, cols, rows, rpc);
+    column_sums_partial_kernel<<<grid, 128, 0, st>>>(ws, m, ld, cols, rows, rpc, map);
     column_sums_reduce_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, st>>>(out, ws, cols, chunks, scale);
     count_launch(2);
     B2_CUDA(cudaGetLastError());

@@ -60,7 +60,7 @@ struct LstmLayerImpl {
     void destroy();
     LstmShape shape() const;
     int load_sequences(int cur_max, int cur_min, const char *pat_dev);
-    // the real frames of the loaded fraction (device list): the products leave out its padding frames
+    // the real frames of the loaded fraction (device list), where the products are to leave out its padding frames; NULL: they are not
     void set_real_frames(const int *map, int n);
     int forward(const float *w, const float *x, float *y, cudaStream_t st);
     int backward(const float *w, const float *x, const float *y, const float *dy, float *dx, float *dw,

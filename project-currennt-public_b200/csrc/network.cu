@@ -126,6 +126,8 @@ int FeedForwardLayer::computeForwardPass(int) {
 
 int FeedForwardLayer::computeBackwardPass(int) {
     const int N = curMax_ * P_, pls = prev_->size(), ls = size_;
+    // padding frames have no error: the products and the sum run over the list of real frames, where the fraction has one
+    const int *real = net_.frac.realMap, NR = real ? (int)net_.frac.realFrames : N;
     {
         ProfScope ps(net_, "ff_delta");
         B2_TRY(ff_delta(outputErrors_, outputs_, (size_t)N * ls, act_, net_.stream));
@@ -135,24 +137,27 @@ int FeedForwardLayer::computeBackwardPass(int) {
         // dX(pls x N) = W delta, overwrite (assignProduct, FeedForwardLayer.cu:1690); nobody reads the
         // errors of an input layer, so that product is skipped
         const bool wantDx = prev_->precedingLayer() != nullptr;
-        const bool tc = !net_.forceFfma && gemm_wants_tc(1, pls, ls, 1, pls, ls, N) &&
-                        (!wantDx || gemm_wants_tc(1, pls, 1, ls, pls, N, ls));
+        const bool tc = !net_.forceFfma && gemm_wants_tc(1, pls, ls, 1, pls, ls, NR) &&
+                        (!wantDx || gemm_wants_tc(1, pls, 1, ls, pls, NR, ls));
         if (tc) {
             // both products on the tensor cores: every operand is split into hi/lo parts ONCE; the deltas' [frame][unit]
             // copy serves as the K-major operand of dX and as the MN-major operand of dW
             TcScratch &sc = net_.tcScratch;
-            B2_TRY(sc.reserve(split_floats(N, ls) + split_floats(N, pls) + split_floats(ls, pls)));
+            B2_TRY(sc.reserve(split_floats(NR, ls) + split_floats(NR, pls) + split_floats(ls, pls)));
             sc.used = 0;
             SplitOperand sD{}, sX{}, sW{};
-            const SplitJob jobs[3] = {{outputErrors_, ls, N, ls, true, 0.0f, &sD}, {prev_->outputs(), pls, N, pls, false, prev_->outputBound(), &sX},
-                                      {weights_, pls, ls, pls, false, 0.0f, &sW}};
+            SplitJob jobs[3] = {{outputErrors_, ls, NR, ls, true, 0.0f, &sD}, {prev_->outputs(), pls, NR, pls, false, prev_->outputBound(), &sX},
+                                {weights_, pls, ls, pls, false, 0.0f, &sW}};
+            jobs[0].map = jobs[1].map = real;
             B2_TRY(split_operands(sc, jobs, wantDx ? 3 : 2, net_.stream));
-            if (wantDx)
-                B2_TRY(gemm_tc(prev_->outputErrors(), pls, sW, sD, pls, N, ls, false, net_.ws, net_.wsFloats, net_.statusDev,
-                               net_.stream));
+            if (wantDx) {
+                B2_TRY(gemm_tc(prev_->outputErrors(), pls, sW, sD, pls, NR, ls, false, net_.ws, net_.wsFloats, net_.statusDev,
+                               net_.stream, real));
+                if (real) B2_TRY(zero_padding_rows(prev_->outputErrors(), pls, pat_, N, net_.stream));
+            }
             SplitOperand sDt = sD;
             sDt.kmajor = false;
-            B2_TRY(gemm_tc(weightUpdates_, pls, sX, sDt, pls, ls, N, false, net_.ws, net_.wsFloats, net_.statusDev, net_.stream));
+            B2_TRY(gemm_tc(weightUpdates_, pls, sX, sDt, pls, ls, NR, false, net_.ws, net_.wsFloats, net_.statusDev, net_.stream));
         } else {
             if (wantDx)
                 B2_TRY(net_.gemm(prev_->outputErrors(), pls, weights_, 1, pls, outputErrors_, 1, ls, pls, N, ls, false));
@@ -162,8 +167,8 @@ int FeedForwardLayer::computeBackwardPass(int) {
     }
     ProfScope ps(net_, "ff_bias_grad");
     // bias gradient = bias * sum over frames of delta (FeedForwardLayer.cu:118-138,1517-1533)
-    return column_sums(weightUpdates_ + (size_t)ls * pls, outputErrors_, ls, ls, N, bias_, net_.ws, net_.wsFloats,
-                       net_.stream);
+    return column_sums(weightUpdates_ + (size_t)ls * pls, outputErrors_, ls, ls, NR, bias_, net_.ws, net_.wsFloats,
+                       net_.stream, real);
 }
 
 // ---- LstmLayer ------------------------------------------------------------------------------------------
@@ -445,7 +450,13 @@ int NeuralNetwork::stageFraction(int b, int T, int nSeq, const int *lens, const 
     B2_CUDA(cudaMemcpyAsync(tgBuf[b], tg, frames * layers.back()->size() * sizeof(float), kind, st));
     Fraction &f = fracBuf[b];
     f.T = mx; f.Tmin = mn; f.nSeq = nSeq; f.realFrames = real;
-    f.patTypes = patBuf[b]; f.realMap = mapBuf[b]; f.inputs = inBuf[b]; f.targets = tgBuf[b];
+    // The products and the sums over frames leave out padding frames where there are enough of them: the launch that zeroes the padding rows
+    // of an error costs what 1000 frames cost in a layer, and the list costs the operand splits and the stores of C a load per row, a few
+    // per cent.  256 sequences of 600 to 1000 frames, 3 blstm layers of 512 units: products, splits and sums over frames 55.5 -> 44.8 ms;
+    // 32 sequences, 2 feed-forward layers of 512 units: their gradients 511 -> 424 us; 4 sequences, 1800 of 4800 frames padding: 2 % of a step.
+    const long pad = (long)frames - real;
+    f.realMap = pad >= 1024 && pad >= (long)frames / 16 ? mapBuf[b] : nullptr;
+    f.patTypes = patBuf[b]; f.inputs = inBuf[b]; f.targets = tgBuf[b];
     return B2_OK;
 }
 

@@ -24,7 +24,7 @@ struct Fraction {
     int T = 0, Tmin = 0, nSeq = 0;
     long realFrames = 0;
     const char *patTypes = nullptr;   // device
-    const int *realMap = nullptr;     // device: frame numbers of the real frames
+    const int *realMap = nullptr;     // device: frame numbers of the real frames; NULL: too few padding frames to leave them out
     const float *inputs = nullptr;    // device, [T*P*inputSize]
     const float *targets = nullptr;   // device, [T*P*outputSize]
 };

@@ -581,11 +581,12 @@ def test_wide_recurrence(els, bi, P, T):
             assert np.array_equal(np.asarray(got[key]), np.asarray(again[key])), "not deterministic: " + key
 
 
-@pytest.mark.parametrize("els,bi,P,T,lo,ff", [(64, 1, 9, 60, 1, 0), (72, 0, 17, 70, 3, 40), (128, 1, 32, 40, 20, 24), (100, 1, 5, 90, 1, 33),
-                                              (256, 0, 3, 300, 2, 0), (600, 1, 20, 13, 1, 30)])
+@pytest.mark.parametrize("els,bi,P,T,lo,ff", [(64, 1, 90, 100, 1, 0), (72, 0, 17, 540, 3, 40), (128, 1, 130, 70, 1, 150), (100, 1, 60, 150, 1, 133),
+                                              (48, 0, 300, 30, 1, 80)])
 def test_products_without_padding_frames(els, bi, P, T, lo, ff):
-    """Ragged fractions whose products run over the list of real frames: operand gathers, the shifted gather of the recurrent weight
-    gradient (tensor-core and FFMA unit counts), results scattered back, zeros at the padding frames below a feed-forward layer."""
+    """Ragged fractions with enough padding frames that the products run over the list of real frames: operand gathers, the shifted
+    gather of the recurrent weight gradient (tensor-core and FFMA unit counts), results scattered back, zeros at the padding frames
+    of a preceding layer's errors; lengths as kernel arguments, or copied (300 sequences)."""
     from b2lstm import workloads
     ls = els * (2 if bi else 1)
     kind = "blstm" if bi else "lstm"
@@ -594,6 +595,7 @@ def test_products_without_padding_frames(els, bi, P, T, lo, ff):
     r = np.random.RandomState(els)
     lens = r.randint(lo, T + 1, P).astype(np.int32)      # in no order
     lens[P // 2], lens[-1] = T, lo
+    assert P * T - lens.sum() >= 4096
     x, tg = workloads.make_fraction(70, 9, P, lens, 95, 96)
     w = workloads.make_weights(layers, 97, 0.08)
     want = run_kind(checker(), layers, P, lens, x, tg, w)
