@@ -139,11 +139,12 @@ int sgd_update(float *w, float *g, float *delta, size_t n, float lr, float mom, 
 // accumulates the AdaGrad statistics, 5 Adam; stats holds n floats (2n for Adam)
 int sgd_update_opt(float *w, float *g, float *delta, float *stats, size_t n, float lr, float mom, int option,
                    const float *frac_len_dev, float beta1_accum, float beta2_accum, cudaStream_t st);
-// pattern types and list of the real frames of a fraction from its sequence lengths (lens: P lengths, P running sums, on the device)
-int fraction_maps(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st);
+// pattern types of a fraction and list of the frames the recurrence runs, t < max(length, tmin), from the sequence lengths (lens: P lengths,
+// 0 for slots without a sequence, and P places in the list where a slot's frames start, on the device)
+int fraction_maps(const int *lens, int P, int tmin, int frames, char *pat, int *map, cudaStream_t st);
 // the same with the lengths in host memory, up to MAX_ARG_LENS sequences
 constexpr int MAX_ARG_LENS = 256;
-int fraction_maps_args(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st);
+int fraction_maps_args(const int *lens, int P, int tmin, int frames, char *pat, int *map, cudaStream_t st);
 // zeroes the rows of m(frames x cols) that belong to padding frames
 int zero_padding_rows(float *m, int cols, const char *pat, int frames, cudaStream_t st);
 int fill_value(float *p, size_t n, float v, cudaStream_t st);
@@ -171,8 +172,8 @@ int lstm_backward_stepwise(const LstmShape &s, const LstmBuffers &b, const float
                            cudaStream_t st);
 // transpose the recurrent block of the weight vector into LstmBuffers::wrecT
 int lstm_prepare_wrecT(const LstmShape &s, const float *w, float *wrecT, cudaStream_t st);
-// bias and peephole gradients (the vector part of the weight update), written into dw; real: the frames to sum over (NULL: all)
-int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *real, int n_real, float *dw, float *ws, size_t ws_floats,
+// bias and peephole gradients (the vector part of the weight update), written into dw; list: the frames to sum over (NULL: all)
+int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *list, int n_list, float *dw, float *ws, size_t ws_floats,
                       cudaStream_t st);
 
 // tensor-core recurrence for large batches (lstm_step_tc.cu): one batched tcgen05 GEMM + one gate

@@ -270,24 +270,24 @@ int accumulate(float *acc, const float *g, size_t n, bool first, cudaStream_t st
     return B2_OK;
 }
 
-// Pattern types of a fraction (1 first, 2 inner, 3 last frame of a sequence, 0 padding) and the list of its real frames, sequence by
-// sequence; one thread per frame.  lens[0..P) are the lengths, lens[P..2P) their running sums.
+// Pattern types of a fraction (1 first, 2 inner, 3 last frame of a sequence, 0 padding) and the list of the frames the recurrence
+// runs (those below tmin in every slot), slot by slot; one thread per frame.  lens[0..P) are the lengths, lens[P..2P) where a slot's frames start.
 namespace {
-struct FractionLens { int len[MAX_ARG_LENS], sum[MAX_ARG_LENS]; };
+struct FractionLens { int len[MAX_ARG_LENS], at[MAX_ARG_LENS]; };
 // few sequences: the lengths come as kernel arguments, which saves the copy
-__global__ void fraction_args_kernel(const __grid_constant__ FractionLens l, int P, int frames, char *__restrict__ pat, int *__restrict__ map) {
+__global__ void fraction_args_kernel(const __grid_constant__ FractionLens l, int P, int tmin, int frames, char *__restrict__ pat, int *__restrict__ map) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= frames) return;
     const int t = f / P, p = f - t * P, len = l.len[p];
     pat[f] = t >= len ? PAT_NONE : (t == 0 ? 1 : (t == len - 1 ? 3 : 2));
-    if (t < len) map[l.sum[p] + t] = f;
+    if (t < max(len, tmin)) map[l.at[p] + t] = f;
 }
-__global__ void fraction_kernel(const int *__restrict__ lens, int P, int frames, char *__restrict__ pat, int *__restrict__ map) {
+__global__ void fraction_kernel(const int *__restrict__ lens, int P, int tmin, int frames, char *__restrict__ pat, int *__restrict__ map) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= frames) return;
     const int t = f / P, p = f - t * P, len = __ldg(lens + p);
     pat[f] = t >= len ? PAT_NONE : (t == 0 ? 1 : (t == len - 1 ? 3 : 2));
-    if (t < len) map[__ldg(lens + P + p) + t] = f;
+    if (t < max(len, tmin)) map[__ldg(lens + P + p) + t] = f;
 }
 __global__ void zero_padding_kernel(float *__restrict__ m, int cols, const char *__restrict__ pat, int frames) {
     for (int f = blockIdx.x * 8 + (int)(threadIdx.x >> 5); f < frames; f += gridDim.x * 8)
@@ -295,16 +295,16 @@ __global__ void zero_padding_kernel(float *__restrict__ m, int cols, const char 
             for (int c = threadIdx.x & 31; c < cols; c += 32) m[(size_t)f * cols + c] = 0.0f;
 }
 }  // namespace
-int fraction_maps(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st) {
-    fraction_kernel<<<(frames + 255) / 256, 256, 0, st>>>(lens, P, frames, pat, map);
+int fraction_maps(const int *lens, int P, int tmin, int frames, char *pat, int *map, cudaStream_t st) {
+    fraction_kernel<<<(frames + 255) / 256, 256, 0, st>>>(lens, P, tmin, frames, pat, map);
     count_launch();
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }
-int fraction_maps_args(const int *lens, int P, int frames, char *pat, int *map, cudaStream_t st) {
+int fraction_maps_args(const int *lens, int P, int tmin, int frames, char *pat, int *map, cudaStream_t st) {
     FractionLens l;
-    for (int p = 0; p < P; ++p) { l.len[p] = lens[p]; l.sum[p] = lens[P + p]; }
-    fraction_args_kernel<<<(frames + 255) / 256, 256, 0, st>>>(l, P, frames, pat, map);
+    for (int p = 0; p < P; ++p) { l.len[p] = lens[p]; l.at[p] = lens[P + p]; }
+    fraction_args_kernel<<<(frames + 255) / 256, 256, 0, st>>>(l, P, tmin, frames, pat, map);
     count_launch();
     B2_CUDA(cudaGetLastError());
     return B2_OK;

@@ -116,14 +116,14 @@ int LstmLayerImpl::load_sequences(int cur_max, int cur_min, const char *pat) {
             return B2_ERR_BAD_ARG;
         }
     }
-    T = cur_max; Tmin = cur_min; bufs.pat = pat; real = nullptr; n_real = 0;
+    T = cur_max; Tmin = cur_min; bufs.pat = pat; list = nullptr; n_list = 0;
     forward_done = false;
     return B2_OK;
 }
 
-void LstmLayerImpl::set_real_frames(const int *map, int n) {
-    real = map;
-    n_real = map ? n : 0;
+void LstmLayerImpl::set_frame_list(const int *map, int n) {
+    list = map;
+    n_list = map ? n : 0;
 }
 
 int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_t st) {
@@ -135,14 +135,14 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
     // LstmLayer.cu:1756-1775): acts(4ls x N) = W_in^T X, W_in viewed as ONE pls x 4ls matrix
     {
         Phase ph(*this, "lstm_proj_gemm");
-        if (real && !force_ffma && scratch && gemm_wants_tc(pls, 1, 1, pls, 4 * ls, n_real, pls)) {
-            B2_TRY(scratch->reserve(split_floats(4 * ls, pls) + split_floats(n_real, pls)));
+        if (list && !force_ffma && scratch && gemm_wants_tc(pls, 1, 1, pls, 4 * ls, n_list, pls)) {
+            B2_TRY(scratch->reserve(split_floats(4 * ls, pls) + split_floats(n_list, pls)));
             scratch->used = 0;
             SplitOperand sW{}, sX{};
-            SplitJob jobs[2] = {{w, pls, 4 * ls, pls, true, 0.0f, &sW}, {x, pls, n_real, pls, true, x_bound, &sX}};
-            jobs[1].map = real;
+            SplitJob jobs[2] = {{w, pls, 4 * ls, pls, true, 0.0f, &sW}, {x, pls, n_list, pls, true, x_bound, &sX}};
+            jobs[1].map = list;
             B2_TRY(split_operands(*scratch, jobs, 2, st));
-            B2_TRY(gemm_tc(bufs.acts, 4 * ls, sW, sX, 4 * ls, n_real, pls, false, ws, ws_floats, status_dev, st, real));
+            B2_TRY(gemm_tc(bufs.acts, 4 * ls, sW, sX, 4 * ls, n_list, pls, false, ws, ws_floats, status_dev, st, list));
         } else {
             B2_TRY(gemm_auto(bufs.acts, 4 * ls, w, pls, 1, x, 1, pls, 4 * ls, N, pls, false, force_ffma, scratch, ws, ws_floats, status_dev,
                              st, x_bound));
@@ -222,11 +222,11 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
         if (rc == 1) { rc = lstm_backward_stepwise(s, bufs, w, dy, st); bwd_path = 0; }
         B2_TRY(rc);
     }
-    const int NR = real ? n_real : N;      // frames the products run over
+    const int NR = list ? n_list : N;      // frames the products run over
     const bool tc = !force_ffma && scratch && gemm_wants_tc(1, pls, 4 * ls, 1, pls, 4 * ls, NR);
-    // contraction length of the recurrent weight gradients: the list of real frames pairs every delta with the h of the step before (its
+    // contraction length of the recurrent weight gradients: the list of frames pairs every delta with the h of the step before (its
     // operand is gathered with a shift), the frames in their order pair all but one timestep
-    const int K = tc && real ? NR : N - P;
+    const int K = tc && list ? NR : N - P;
     SplitOperand sD{}, sX{}, sY{}, sW{};
     if (tc) {
         // every operand of the four contractions is split into hi/lo parts ONCE and reused:
@@ -238,8 +238,8 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
         // the gate deltas are clipped to [-1, 1] (helpers/limitedError.cuh of the reference), |h| = |tanh(c) * og| < 1
         SplitJob jobs[4] = {{bufs.deltas, 4L * ls, NR, 4 * ls, true, 1.0f, &sD}, {y, ls, NR, ls, false, 1.0f, &sY},
                             {x, pls, NR, pls, false, x_bound, &sX}, {w, pls, 4 * ls, pls, false, 0.0f, &sW}};
-        if (real) {
-            jobs[0].map = jobs[1].map = jobs[2].map = real;
+        if (list) {
+            jobs[0].map = jobs[1].map = jobs[2].map = list;
             // h of the previous step in sweep order: a timestep below for the forward direction, above for the other
             jobs[1].shift = P; jobs[1].shift_cols = els; jobs[1].src_rows = N;
         }
@@ -251,8 +251,8 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
         if (tc) {
             SplitOperand A = sW, B = sD;
             A.kmajor = false; B.kmajor = true;
-            B2_TRY(gemm_tc(dx, pls, A, B, pls, NR, 4 * ls, false, ws, ws_floats, status_dev, st, real));
-            if (real) B2_TRY(zero_padding_rows(dx, pls, bufs.pat, N, st));
+            B2_TRY(gemm_tc(dx, pls, A, B, pls, NR, 4 * ls, false, ws, ws_floats, status_dev, st, list));
+            if (list) B2_TRY(zero_padding_rows(dx, pls, bufs.pat, N, st));
         } else {
             B2_TRY(gemm(dx, pls, w, 1, pls, bufs.deltas, 1, 4 * ls, pls, N, 4 * ls, false, st));
         }
@@ -303,8 +303,8 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
                 for (int d = 0; d < D; ++d)
                     for (int g = 0; g < 4; ++g) {
                         TcBatch &b = bt[d * 4 + g];
-                        b.a_in = d * els; b.a_out = d && !real ? P : 0;        // h of the previous step in sweep order
-                        b.b_in = g * ls + d * els; b.b_out = d || real ? 0 : P;
+                        b.a_in = d * els; b.a_out = d && !list ? P : 0;        // h of the previous step in sweep order
+                        b.b_in = g * ls + d * els; b.b_out = d || list ? 0 : P;
                         coff[d * 4 + g] = (long long)(off.rec + ((size_t)g * ls + (size_t)d * els) * els);
                         b.c_off = splits > 1 ? (long long)(d * 4 + g) * splits * (long long)per : coff[d * 4 + g];
                     }
@@ -325,7 +325,7 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
             }
     }
     Phase ph(*this, "lstm_vector_grads");
-    B2_TRY(lstm_vector_grads(s, bufs, real, n_real, dw, ws, ws_floats, st));
+    B2_TRY(lstm_vector_grads(s, bufs, list, n_list, dw, ws, ws_floats, st));
     return B2_OK;
 }
 

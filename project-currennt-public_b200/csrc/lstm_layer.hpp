@@ -15,8 +15,8 @@ struct LstmLayerImpl {
     bool check_padding = false;   // load_sequences verifies that padding frames trail their sequences
     int *pad_dev = nullptr;       // result word of that check
     LstmBuffers bufs{};
-    const int *real = nullptr;    // the real frames of the fraction, n_real of them (NULL: the products take all frames)
-    int n_real = 0;
+    const int *list = nullptr;    // the frames of the fraction the sweeps run, n_list of them (NULL: the products take all frames)
+    int n_list = 0;
     float *ws = nullptr;       // scratch: split-K partials, vector-gradient partials
     size_t ws_floats = 0;
     size_t state_bytes = 0;
@@ -60,8 +60,9 @@ struct LstmLayerImpl {
     void destroy();
     LstmShape shape() const;
     int load_sequences(int cur_max, int cur_min, const char *pat_dev);
-    // the real frames of the loaded fraction (device list), where the products are to leave out its padding frames; NULL: they are not
-    void set_real_frames(const int *map, int n);
+    // The frames of the loaded fraction that the sweeps run (device list: t below the slot's length or the shortest one), where the products
+    // are to leave out the others; NULL: they are not.  A frame that is missing keeps stale pre-activations: the list must hold every such frame.
+    void set_frame_list(const int *map, int n);
     int forward(const float *w, const float *x, float *y, cudaStream_t st);
     int backward(const float *w, const float *x, const float *y, const float *dy, float *dx, float *dw,
                  cudaStream_t st);

@@ -208,18 +208,18 @@ __global__ void wrec_transpose_kernel(int ls, int els, int D, const float *__res
 // Bias and peephole gradients: per unit u and frame chunk, partial sums of
 //   delta_g[f][u] (4 gates), c[f -/+ P]*delta_ig/fg[f] and c[f]*delta_og[f]
 // (layers/LstmLayer.cu:524-541,574-610 of the reference), then a fixed-order reduction.
-__global__ void lstm_vgrad_partial_kernel(LstmShape sh, LstmBuffers bf, const int *__restrict__ real, int n_real, float *__restrict__ ws,
+__global__ void lstm_vgrad_partial_kernel(LstmShape sh, LstmBuffers bf, const int *__restrict__ list, int n_list, float *__restrict__ ws,
                                           int frames_per_chunk) {
     const int ls = sh.ls, els = sh.els, P = sh.P;
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= ls) return;
     const int d = u / els;
-    const long N = (long)sh.T * P, frames = real ? n_real : N;      // padding frames add nothing
+    const long N = (long)sh.T * P, frames = list ? n_list : N;      // padding frames add nothing
     const long i0 = (long)blockIdx.y * frames_per_chunk, i1 = min(frames, i0 + frames_per_chunk);
     float s[7] = {0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
     for (long i = i0; i < i1; ++i) {
-        const long f = real ? __ldg(real + i) : i;
+        const long f = list ? __ldg(list + i) : i;
         const float *dl = bf.deltas + (size_t)f * 4 * ls + u;
         float dni = dl[0], dig = dl[ls], dfg = dl[2 * ls], dog = dl[3 * ls];
         s[0] += dni; s[1] += dig; s[2] += dfg; s[3] += dog;
@@ -285,9 +285,9 @@ int lstm_backward_stepwise(const LstmShape &s, const LstmBuffers &b, const float
     return B2_OK;
 }
 
-int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *real, int n_real, float *dw, float *ws, size_t ws_floats,
+int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *list, int n_list, float *dw, float *ws, size_t ws_floats,
                       cudaStream_t st) {
-    const long N = real ? n_real : (long)s.T * s.P;
+    const long N = list ? n_list : (long)s.T * s.P;
     // chunks of frames: enough blocks to fill the device several times over, bounded by the scratch
     // (800 frames x 128 units, 64 frames a chunk: 13 blocks, each a chain of 16 rounds of loads)
     long fit = N * ((s.ls + 127) / 128) / (4 * sm_count());
@@ -300,7 +300,7 @@ int lstm_vector_grads(const LstmShape &s, const LstmBuffers &b, const int *real,
     if ((N + fpc - 1) / fpc > max_chunks) fpc = (int)((N + max_chunks - 1) / max_chunks);
     int chunks = (int)((N + fpc - 1) / fpc);
     dim3 grid((s.ls + 127) / 128, chunks);
-    lstm_vgrad_partial_kernel<<<grid, 128, 0, st>>>(s, b, real, n_real, ws, fpc);
+    lstm_vgrad_partial_kernel<<<grid, 128, 0, st>>>(s, b, list, n_list, ws, fpc);
     lstm_vgrad_reduce_kernel<<<(7 * s.ls + 31) / 32, dim3(32, 8), 0, st>>>(s, chunks, ws, dw);
     count_launch(2);
     B2_CUDA(cudaGetLastError());

@@ -126,8 +126,8 @@ int FeedForwardLayer::computeForwardPass(int) {
 
 int FeedForwardLayer::computeBackwardPass(int) {
     const int N = curMax_ * P_, pls = prev_->size(), ls = size_;
-    // padding frames have no error: the products and the sum run over the list of real frames, where the fraction has one
-    const int *real = net_.frac.realMap, NR = real ? (int)net_.frac.realFrames : N;
+    // padding frames have no error: the products and the sum run over the list of frames, where the fraction has one
+    const int *list = net_.frac.frameList, NR = list ? net_.frac.listFrames : N;
     {
         ProfScope ps(net_, "ff_delta");
         B2_TRY(ff_delta(outputErrors_, outputs_, (size_t)N * ls, act_, net_.stream));
@@ -148,12 +148,12 @@ int FeedForwardLayer::computeBackwardPass(int) {
             SplitOperand sD{}, sX{}, sW{};
             SplitJob jobs[3] = {{outputErrors_, ls, NR, ls, true, 0.0f, &sD}, {prev_->outputs(), pls, NR, pls, false, prev_->outputBound(), &sX},
                                 {weights_, pls, ls, pls, false, 0.0f, &sW}};
-            jobs[0].map = jobs[1].map = real;
+            jobs[0].map = jobs[1].map = list;
             B2_TRY(split_operands(sc, jobs, wantDx ? 3 : 2, net_.stream));
             if (wantDx) {
                 B2_TRY(gemm_tc(prev_->outputErrors(), pls, sW, sD, pls, NR, ls, false, net_.ws, net_.wsFloats, net_.statusDev,
-                               net_.stream, real));
-                if (real) B2_TRY(zero_padding_rows(prev_->outputErrors(), pls, pat_, N, net_.stream));
+                               net_.stream, list));
+                if (list) B2_TRY(zero_padding_rows(prev_->outputErrors(), pls, pat_, N, net_.stream));
             }
             SplitOperand sDt = sD;
             sDt.kmajor = false;
@@ -168,7 +168,7 @@ int FeedForwardLayer::computeBackwardPass(int) {
     ProfScope ps(net_, "ff_bias_grad");
     // bias gradient = bias * sum over frames of delta (FeedForwardLayer.cu:118-138,1517-1533)
     return column_sums(weightUpdates_ + (size_t)ls * pls, outputErrors_, ls, ls, NR, bias_, net_.ws, net_.wsFloats,
-                       net_.stream, real);
+                       net_.stream, list);
 }
 
 // ---- LstmLayer ------------------------------------------------------------------------------------------
@@ -197,7 +197,7 @@ int LstmLayer::init() {
 int LstmLayer::loadSequences(const Fraction &f, int nnState) {
     Layer::loadSequences(f, nnState);
     B2_TRY(impl_.load_sequences(f.T, f.Tmin, f.patTypes));
-    impl_.set_real_frames(f.realMap, (int)f.realFrames);
+    impl_.set_frame_list(f.frameList, f.listFrames);
     return B2_OK;
 }
 int LstmLayer::computeForwardPass(int) {
@@ -433,17 +433,20 @@ int NeuralNetwork::stageFraction(int b, int T, int nSeq, const int *lens, const 
     int la[2 * MAX_ARG_LENS], *lh = args ? la : lenPinned[b];
     // the pinned staging is rewritten by the host: the previous copy out of it must have run
     if (!args) B2_CUDA(cudaEventSynchronize(patCopied[b]));
-    for (int p = 0, sum = 0; p < P; ++p) {
+    // The list holds every frame the recurrence runs: below the shortest length the frames of EVERY slot, those without a sequence
+    // included (the reference looks at the pattern types from the shortest length on only, layers/LstmLayer.cu:89-101).
+    long listed = 0;
+    for (int p = 0; p < P; ++p) {
         lh[p] = p < nSeq ? lens[p] : 0;
-        lh[P + p] = sum;
-        sum += lh[p];
+        lh[P + p] = (int)listed;
+        listed += lh[p] > mn ? lh[p] : mn;
     }
     if (args) {
-        B2_TRY(fraction_maps_args(lh, P, (int)frames, patBuf[b], mapBuf[b], st));
+        B2_TRY(fraction_maps_args(lh, P, mn, (int)frames, patBuf[b], mapBuf[b], st));
     } else {
         B2_CUDA(cudaMemcpyAsync(lenBuf[b], lh, (size_t)2 * P * sizeof(int), cudaMemcpyHostToDevice, st));
         B2_CUDA(cudaEventRecord(patCopied[b], st));
-        B2_TRY(fraction_maps(lenBuf[b], P, (int)frames, patBuf[b], mapBuf[b], st));
+        B2_TRY(fraction_maps(lenBuf[b], P, mn, (int)frames, patBuf[b], mapBuf[b], st));
     }
     cudaMemcpyKind kind = onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     B2_CUDA(cudaMemcpyAsync(inBuf[b], in, frames * layers.front()->size() * sizeof(float), kind, st));
@@ -454,8 +457,9 @@ int NeuralNetwork::stageFraction(int b, int T, int nSeq, const int *lens, const 
     // of an error costs what 1000 frames cost in a layer, and the list costs the operand splits and the stores of C a load per row, a few
     // per cent.  256 sequences of 600 to 1000 frames, 3 blstm layers of 512 units: products, splits and sums over frames 55.5 -> 44.8 ms;
     // 32 sequences, 2 feed-forward layers of 512 units: their gradients 511 -> 424 us; 4 sequences, 1800 of 4800 frames padding: 2 % of a step.
-    const long pad = (long)frames - real;
-    f.realMap = pad >= 1024 && pad >= (long)frames / 16 ? mapBuf[b] : nullptr;
+    const long pad = (long)frames - listed;
+    f.frameList = pad >= 1024 && pad >= (long)frames / 16 ? mapBuf[b] : nullptr;
+    f.listFrames = (int)listed;
     f.patTypes = patBuf[b]; f.inputs = inBuf[b]; f.targets = tgBuf[b];
     return B2_OK;
 }

@@ -24,7 +24,8 @@ struct Fraction {
     int T = 0, Tmin = 0, nSeq = 0;
     long realFrames = 0;
     const char *patTypes = nullptr;   // device
-    const int *realMap = nullptr;     // device: frame numbers of the real frames; NULL: too few padding frames to leave them out
+    const int *frameList = nullptr;   // device: the listFrames frames the recurrence runs; NULL: too few others to leave them out
+    int listFrames = 0;
     const float *inputs = nullptr;    // device, [T*P*inputSize]
     const float *targets = nullptr;   // device, [T*P*outputSize]
 };
@@ -188,7 +189,7 @@ public:
     // (on copyStream) while the current one is being processed
     float *inBuf[2] = {nullptr, nullptr}, *tgBuf[2] = {nullptr, nullptr};
     char *patBuf[2] = {nullptr, nullptr};
-    int *mapBuf[2] = {nullptr, nullptr};       // the real frames of the fraction
+    int *mapBuf[2] = {nullptr, nullptr};       // list of the frames the recurrence runs
     int *lenBuf[2] = {nullptr, nullptr};       // sequence lengths and their running sums
     int *lenPinned[2] = {nullptr, nullptr};    // ... pinned host staging (both only for more than MAX_ARG_LENS sequences)
     Fraction fracBuf[2];

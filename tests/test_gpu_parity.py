@@ -615,3 +615,42 @@ def test_recurrent_weight_gradient_with_splits_of_whole_slabs():
     want = run_kind(checker(), layers, 4, lens, x, tg, w)
     got = run_gpu(layers, 4, lens, x, tg, w, VARIANTS[2])
     parity.compare_run(layers, got, want, "4 x 400", lstm_pad_zero_lens=lens)
+
+
+@pytest.mark.parametrize("P,lens,bi,els", [(64, [60, 57, 41, 33, 20], 1, 64), (64, [60, 20], 0, 300), (300, [60, 57, 50, 41, 33, 20], 1, 48)])
+def test_empty_slots_of_a_later_fraction(P, lens, bi, els):
+    """A fraction with fewer sequences than the net has slots and enough padding that the products run over a list of frames, the second
+    one on its net: frames below the shortest length are real in EVERY slot (layers/LstmLayer.cu:89-101), empty ones included, so
+    their outputs must not depend on what the fraction before left behind.  Lengths as kernel arguments, or copied (300 slots)."""
+    import b2lstm
+    from b2lstm import workloads
+    kind, ls = ("blstm", 2 * els) if bi else ("lstm", els)
+    layers = L(("input", 70), ("feedforward_tanh", 72), (kind, ls), (kind, ls), ("feedforward_identity", 9), ("sse", 9))
+    w = workloads.make_weights(layers, 101, 0.08)
+    first, lens = np.full(P, 60, np.int32), np.array(lens, np.int32)
+    fractions = [(first, workloads.make_fraction(70, 9, P, first, 102, 103)), (lens, workloads.make_fraction(70, 9, P, lens, 104, 105))]
+    T = int(lens.max())
+    swept = sum(max(int(lens[p]) if p < len(lens) else 0, int(lens.min())) for p in range(P))
+    assert T * P - swept >= max(1024, T * P // 16)
+    want = run_kind(checker(), layers, P, lens, fractions[1][1][0], fractions[1][1][1], w)
+
+    def results(net):
+        got = {"loss": net.forward()}
+        net.backward()
+        for i in range(1, 5):
+            got["out%d" % i] = net.outputs(i)
+            got["dw%d" % i] = net.weight_updates(i)
+        return got
+    runs = []
+    for k in (0, 1):
+        net = b2lstm.Net(layers, P, 60)
+        for i, wi in w.items():
+            net.set_weights(i, wi)
+        for f in fractions[k:]:
+            net.load_fraction(f[0], *f[1])
+            got = results(net)
+        runs.append(got)
+        net.close()
+    parity.compare_run(layers, runs[0], want, "P%d, %d sequences" % (P, len(lens)), lstm_pad_zero_lens=lens)
+    for key in runs[0]:
+        assert np.array_equal(np.asarray(runs[0][key]), np.asarray(runs[1][key])), "depends on the fraction before: " + key
