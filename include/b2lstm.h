@@ -287,6 +287,9 @@ int b2_selftest_bounded_wait(int *status_out, int *gave_up);
  * net's kernels record a given-up wait in, exactly where a kernel would have put it (no kernel is made to fail).
  * The next b2_net_synchronize, b2_net_train_epoch or b2_optimizer_train must return `code`. */
 int b2_selftest_inject_status(b2_net *net, int code);
+/* Self-test of the activations of the persistent recurrence kernels: for n host floats x the logistic function, the tanh and
+ * 1 / (1 + |x|) as those kernels compute them on the device (activation_functions/{Logistic,Tanh}.cuh of the reference). */
+int b2_selftest_activations(const float *x, int n, float *logistic, float *tanh, float *rcp);
 
 /* ------------------------------------------------------------------------------------------
  * Data-parallel training: sequences of a fraction are dealt to the ranks, every rank holds a

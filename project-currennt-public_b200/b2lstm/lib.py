@@ -92,6 +92,7 @@ SIGNATURES = {
     "b2_net_get_profile": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_char_p), _fp, _ip]),
     "b2_selftest_bounded_wait": (C.c_int, [_ip, _ip]),
     "b2_selftest_inject_status": (C.c_int, [C.c_void_p, C.c_int]),
+    "b2_selftest_activations": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     "b2_dp_get_unique_id": (C.c_int, [C.c_void_p]),
     "b2_dp_attach": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p]),
     "b2_dp_detach": (C.c_int, [C.c_void_p]),
@@ -226,6 +227,14 @@ def selftest_bounded_wait():
     st, gu = C.c_int(), C.c_int()
     _check(lib().b2_selftest_bounded_wait(C.byref(st), C.byref(gu)))
     return st.value, bool(gu.value)
+
+
+def selftest_activations(x):
+    """(logistic, tanh, 1 / (1 + |x|)) of a float32 array as the persistent recurrence kernels compute them"""
+    x = np.ascontiguousarray(x, np.float32)
+    out = [np.empty_like(x) for _ in range(3)]
+    _check(lib().b2_selftest_activations(x.ctypes.data, x.size, *[o.ctypes.data for o in out]))
+    return out
 
 
 def dp_unique_id():

@@ -1,4 +1,4 @@
-// What the recurrence kernels on thread-block clusters share (lstm_cluster.cu, lstm_single.cu): activations, bounded waits on
+// What the recurrence kernels on thread-block clusters share (lstm_cluster.cu, lstm_single.cu, lstm_wide.cu): activations, bounded waits on
 // transaction barriers, sequence lengths.
 #pragma once
 #include "common.cuh"
@@ -9,17 +9,20 @@ namespace cluster {
 
 constexpr unsigned SPIN_LIMIT = 1u << 21;
 
-// 1 / d, d >= 1: the hardware approximation and one Newton step (r + r (1 - d r)): as exact as the division, without branches
+// 1 / d, 1 <= d < 2^126: the hardware approximation (relative error e <= 2^-23) and one Newton step (r + r (1 - d r), relative error
+// e^2 before the last rounding): within 0.5001 ulp, without the division's branches
 __device__ __forceinline__ float cl_rcp(float d) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
-// The exponent limits take the place of the reference's cut-offs (activation_functions/Logistic.cuh): below them the quotients
-// are 0 (logistic) and -1 (tanh).  tanh as (1 - e) / (1 + e), e = exp(-2x), loses less than 2 logistic(2x) - 1 does.
-__device__ __forceinline__ float cl_logistic(float x) { return cl_rcp(1.0f + expf(fminf(-x, 88.0f))); }
+// The exponent limits take the place of the reference's cut-offs (activation_functions/Logistic.cuh): above the upper one the quotients
+// are 0 (logistic) and -1 (tanh); the lower one is where a NaN goes, which ends as 1 like there.  tanh as (1 - e) / (1 + e),
+// e = exp(-2x), loses less than 2 logistic(2x) - 1 does.
+__device__ __forceinline__ float cl_exp(float x, float most) { return expf(fminf(fmaxf(x, -88.0f), most)); }
+__device__ __forceinline__ float cl_logistic(float x) { return cl_rcp(1.0f + cl_exp(-x, 88.0f)); }
 __device__ __forceinline__ float cl_tanh(float x) {
-    const float e = expf(fminf(-2.0f * x, 40.0f));
+    const float e = cl_exp(-2.0f * x, 40.0f);
     return (1.0f - e) * cl_rcp(1.0f + e);
 }
 

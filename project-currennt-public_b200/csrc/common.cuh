@@ -244,6 +244,7 @@ int persistent_ps(int els, int P, int D, bool use_cluster);   // sequences per w
 // many items as fit side by side, the remaining sequences through L2 on the SMs the clusters leave free)
 int lstm_persistent(bool backward, int transport, const LstmShape &s, const LstmBuffers &b, const float *w, float *y,
                     const float *dy, unsigned long long *xchg, int *status, unsigned *tag_next, cudaStream_t st);
+int lstm_selftest_activations(const float *x, int n, float *logistic, float *tanh, float *rcp);   // host arrays
 int lstm_selftest_bounded_wait(int *status_out, int *gave_up, cudaStream_t st);
 
 // offsets inside the (b)lstm weight vector

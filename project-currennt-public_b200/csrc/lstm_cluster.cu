@@ -627,6 +627,16 @@ __global__ void __launch_bounds__(32 * WN, 1) lstm_bwd_cluster_kernel(ClusterArg
     }
 }
 
+// x(n) and behind it, for each entry, its logistic, its tanh and 1 / (1 + |x|) as the recurrence kernels compute them
+__global__ void activations_selftest_kernel(float *v, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float x = v[i];
+    v[(size_t)n + i] = cl_logistic(x);
+    v[(size_t)2 * n + i] = cl_tanh(x);
+    v[(size_t)3 * n + i] = cl_rcp(1.0f + fabsf(x));
+}
+
 // ---- host side ---------------------------------------------------------------------------------------------------------------
 typedef void (*Kernel)(ClusterArgs);
 struct Variant {
@@ -756,6 +766,23 @@ Plan make_plan(const LstmShape &s, bool backward) {
 }
 
 }  // namespace
+
+int lstm_selftest_activations(const float *x, int n, float *logistic, float *tanh, float *rcp) {
+    float *dev = nullptr;
+    const size_t bytes = (size_t)n * sizeof(float);
+    B2_CUDA(cudaMalloc(&dev, 4 * bytes));
+    cudaError_t e = cudaMemcpy(dev, x, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        activations_selftest_kernel<<<(n + 255) / 256, 256>>>(dev, n);
+        count_launch();
+        e = cudaGetLastError();
+    }
+    float *const out[3] = {logistic, tanh, rcp};
+    for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMemcpy(out[i], dev + (size_t)(i + 1) * n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(dev);
+    B2_CUDA(e);
+    return B2_OK;
+}
 
 bool lstm_cluster_supported(const LstmShape &s) { return s.els <= 512 && make_plan(s, false).vi >= 0 && make_plan(s, true).vi >= 0; }
 

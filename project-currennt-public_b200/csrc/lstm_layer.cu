@@ -455,6 +455,10 @@ int b2_selftest_bounded_wait(int *status_out, int *gave_up) {
     return b2::lstm_selftest_bounded_wait(status_out, gave_up, nullptr);
 }
 
+int b2_selftest_activations(const float *x, int n, float *logistic, float *tanh, float *rcp) {
+    if (!x || n <= 0 || !logistic || !tanh || !rcp) { b2::set_error("b2_selftest_activations: bad arguments"); return B2_ERR_BAD_ARG; }
+    return b2::lstm_selftest_activations(x, n, logistic, tanh, rcp);
+}
 
 size_t b2_lstm_num_weights(const b2_lstm_desc *d) {
     if (!d) return 0;

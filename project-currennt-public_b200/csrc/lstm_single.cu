@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(NTHR, 1) lstm_fwd_single_kernel(SingleArgs a) 
             }
             // gate 0 tanh, gates 1 and 2 logistic, each in the lanes of its row; gate 3 waits for the new cell state
             const float xp = fmaf(cp, peep, x);
-            const float e = expf(fminf(gate == 0 ? -2.0f * xp : -xp, gate == 0 ? 40.0f : 88.0f)), r = cl_rcp(1.0f + e);
+            const float e = cl_exp(gate == 0 ? -2.0f * xp : -xp, gate == 0 ? 40.0f : 88.0f), r = cl_rcp(1.0f + e);
             float act = gate == 0 ? (1.0f - e) * r : r;
             const float ni = __shfl_sync(0xffffffffu, act, base), ig = __shfl_sync(0xffffffffu, act, base + LPR);
             const float fg = __shfl_sync(0xffffffffu, act, base + 2 * LPR), xo = __shfl_sync(0xffffffffu, x, base + 3 * LPR);

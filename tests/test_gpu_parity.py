@@ -654,3 +654,48 @@ def test_empty_slots_of_a_later_fraction(P, lens, bi, els):
     parity.compare_run(layers, runs[0], want, "P%d, %d sequences" % (P, len(lens)), lstm_pad_zero_lens=lens)
     for key in runs[0]:
         assert np.array_equal(np.asarray(runs[0][key]), np.asarray(runs[1][key])), "depends on the fraction before: " + key
+
+
+@pytest.mark.parametrize("els,bi,P", [(16, 1, 9), (128, 1, 12), (256, 0, 3), (256, 1, 32), (512, 1, 1), (512, 0, 20), (512, 1, 128), (1024, 1, 16),
+                                      (1024, 0, 1)])
+def test_nan_in_a_pre_activation_ends_as_in_the_reference(els, bi, P):
+    """A NaN in one frame of the input makes every pre-activation of that frame NaN.  The reference's cut-offs turn it into 1
+    (activation_functions/Logistic.cuh: no comparison with a NaN holds); every recurrence kernel must do the same."""
+    from b2lstm import workloads
+    ls = els * (2 if bi else 1)
+    layers = L(("input", 7), ("blstm" if bi else "lstm", ls), ("feedforward_identity", 5), ("sse", 5))
+    lens = np.array([6] * P, np.int32)
+    x, tg = workloads.make_fraction(7, 5, P, lens, 111, 112)
+    x[2, P // 2, 3] = np.nan
+    w = workloads.make_weights(layers, 113, 0.2 if els < 100 else 0.08)
+    want = run_kind(checker(), layers, P, lens, x, tg, w)
+    assert np.isfinite(want["out1"]).all()
+    for mode in (1, 0):
+        got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=mode, ffma=0))
+        parity.assert_outputs_close(got["out1"], want["out1"], "mode %d" % mode)
+        assert abs(got["loss"] - want["loss"]) <= 1e-5 * want["loss"], mode
+
+
+def test_activations_of_the_recurrence_kernels():
+    """The kernels' own logistic, tanh and reciprocal against float64.  Reciprocal: half an ulp and e^2 = 2^-46 of the Newton step.
+    Logistic: expf within 2 ulp (relative 2^-22), the sum and the reciprocal half an ulp each: relative 2^-22 + 2^-23.  tanh: the error of
+    e = exp(-2x) moves (1 - e) / (1 + e) by 2 e / (1 + e)^2 <= 1/2 of its relative size, four roundings of 2^-24: 2^-23 + 2^-22 |tanh|.
+    Results below the smallest normal number may come out as 0.  NaN ends as 1, as the reference's cut-offs make it."""
+    from b2lstm.lib import selftest_activations
+    rng = np.random.default_rng(7)
+    x = np.concatenate([rng.uniform(-20, 20, 200000), rng.uniform(-100, 100, 50000), rng.standard_normal(50000) * 1e-3,
+                        10.0 ** rng.uniform(-30, 37, 50000), [0.0, -0.0, 88.0, -88.0, 87.3, -87.3]]).astype(np.float32)
+    log, tanh, rcp = [a.astype(np.float64) for a in selftest_activations(x)]
+    x64 = x.astype(np.float64)
+    with np.errstate(over="ignore"):
+        want = 1.0 / (1.0 + np.exp(-x64))
+    tiny = float(np.finfo(np.float32).tiny)
+    assert (np.abs(log - want) <= (2.0 ** -22 + 2.0 ** -23) * want + 2 * tiny).all()
+    assert (np.abs(tanh - np.tanh(x64)) <= 2.0 ** -23 + 2.0 ** -22 * np.abs(np.tanh(x64))).all()
+    d = np.float32(1.0) + np.abs(x)
+    inv = 1.0 / d.astype(np.float64)
+    ulp = np.spacing(inv.astype(np.float32)).astype(np.float64)
+    print("reciprocal: largest error %.4f ulp" % (np.abs(rcp - inv) / ulp).max())
+    assert (np.abs(rcp - inv) <= 0.5001 * ulp + tiny * (inv < tiny)).all()
+    special = selftest_activations(np.array([np.nan, np.inf, -np.inf, 1e30, -1e30, 200.0, -200.0], np.float32))
+    assert special[0].tolist() == [1, 1, 0, 1, 0, 1, 0] and special[1].tolist() == [1, 1, -1, 1, -1, 1, -1]
