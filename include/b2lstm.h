@@ -137,6 +137,10 @@ int b2_lstm_set_recurrence_mode(b2_lstm *layer, int mode);
  * thread-block clusters; -1 before the first sweep.  The reference
  * has one code path (layers/LstmLayer.cu:1805-1858), so it has no such query. */
 int b2_lstm_recurrence_path(const b2_lstm *layer, int backward);
+/* The same by name, which tells the members of a family apart: the source file of the kernels that ran, "lstm_step" (path 0),
+ * "lstm_persistent" or "lstm_single" (1), "lstm_step_tc" (3), "lstm_ptc" or "lstm_wide" (5), "lstm_cluster" (7); "" before the first
+ * sweep.  The text is static. */
+const char *b2_lstm_recurrence_kernel(const b2_lstm *layer, int backward);
 /* Waits for the work enqueued on `stream` and reports what the layer's kernels recorded:
  * B2_ERR_STEP_TIMEOUT if a persistent kernel gave up a bounded wait, else B2_OK. */
 int b2_lstm_synchronize(b2_lstm *layer, b2_stream stream);
@@ -267,6 +271,8 @@ b2_stream b2_net_stream(b2_net *net);
 int b2_net_set_recurrence_mode(b2_net *net, int mode);
 /* b2_lstm_recurrence_path of layer `layer` of the net; -1 for layers that are no (b)lstm. */
 int b2_net_recurrence_path(b2_net *net, int layer, int backward);
+/* b2_lstm_recurrence_kernel of layer `layer` of the net; "" for layers that are no (b)lstm. */
+const char *b2_net_recurrence_kernel(b2_net *net, int layer, int backward);
 /* Non-zero forces the FFMA GEMM everywhere (the tensor-core GEMM is the default). */
 int b2_net_set_force_ffma(b2_net *net, int on);
 /* Number of kernels this library has launched on behalf of `net` since creation. */

@@ -44,6 +44,8 @@ SIGNATURES = {
     "b2_lstm_state_bytes": (C.c_size_t, [C.c_void_p]),
     "b2_lstm_recurrence_path": (C.c_int, [C.c_void_p, C.c_int]),
     "b2_net_recurrence_path": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
+    "b2_lstm_recurrence_kernel": (C.c_char_p, [C.c_void_p, C.c_int]),
+    "b2_net_recurrence_kernel": (C.c_char_p, [C.c_void_p, C.c_int, C.c_int]),
     "b2_lstm_synchronize": (C.c_int, [C.c_void_p, C.c_void_p]),
     "b2_net_create": (C.c_int, [C.c_char_p, C.c_int, C.c_int, C.c_uint, C.POINTER(C.c_void_p)]),
     "b2_config_set_lstm_forget_gate_bias": (None, [C.c_float]),
@@ -213,6 +215,10 @@ class LstmLayer:
 
     def recurrence_path(self, backward=False):
         return int(lib().b2_lstm_recurrence_path(self.h, int(backward)))
+
+    def recurrence_kernel(self, backward=False):
+        """source file of the kernels the layer's last sweep ran ("" before the first)"""
+        return lib().b2_lstm_recurrence_kernel(self.h, int(backward)).decode()
 
     def set_check_padding(self, on):
         _check(lib().b2_lstm_set_check_padding(self.h, int(on)))
@@ -391,6 +397,15 @@ class Net:
             if f >= 0:
                 b = self.recurrence_path(i, True)
                 out[i] = (self.RECURRENCE_PATHS.get(f, str(f)), self.RECURRENCE_PATHS.get(b, str(b)))
+        return out
+
+    def recurrence_kernels(self):
+        """{layer index: (forward, backward)}: source files of the kernels the (b)lstm layers' last sweeps ran"""
+        out = {}
+        for i in range(int(lib().b2_net_num_layers(self.h))):
+            names = tuple(lib().b2_net_recurrence_kernel(self.h, i, b).decode() for b in (0, 1))
+            if names[0]:
+                out[i] = names
         return out
 
     @property

@@ -156,7 +156,7 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
             const bool single = lstm_single_supported(s, false);
             rc = single ? lstm_single_sweep(false, s, bufs, w, y, nullptr, status_dev, st)
                         : lstm_cluster_sweep(false, s, bufs, w, y, nullptr, status_dev, st);
-            fwd_path = single ? 1 : 7;
+            fwd_path = single ? 1 : 7; fwd_kernel = single ? "lstm_single" : "lstm_cluster";
         }
         wide_used = !cluster_used && want_wide();
         ptc_used = !cluster_used && !wide_used && want_ptc();
@@ -164,13 +164,13 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
             B2_TRY(ensure_ptc());
             B2_TRY(lstm_ptc_prepare(s, w, ptc, st));
             rc = lstm_ptc_sweep(false, s, bufs, ptc, w, y, nullptr, status_dev, &tag_next, st);
-            fwd_path = 5;
+            fwd_path = 5; fwd_kernel = "lstm_ptc";
             if (rc == 1) ptc_used = false;
         }
         if (wide_used) {
             B2_TRY(ensure_wide());
             rc = lstm_wide_sweep(false, s, bufs, wide, w, y, nullptr, status_dev, &tag_next, st);
-            fwd_path = 5;
+            fwd_path = 5; fwd_kernel = "lstm_wide";
         }
         tcrec_used = !cluster_used && !ptc_used && !wide_used && want_tc_recurrence();
         const bool plain = !cluster_used && !ptc_used && !wide_used && !tcrec_used;
@@ -179,12 +179,12 @@ int LstmLayerImpl::forward(const float *w, const float *x, float *y, cudaStream_
         } else if (tcrec_used) {
             B2_TRY(ensure_tcrec());
             rc = lstm_forward_tc(s, bufs, tcrec, w, y, status_dev, st);
-            fwd_path = 3;
+            fwd_path = 3; fwd_kernel = "lstm_step_tc";
         } else if (recurrence_mode >= 1) {
             rc = lstm_persistent(false, persistent_transport(), s, bufs, w, y, nullptr, xchg, status_dev, &tag_next, st);
-            fwd_path = 1;
+            fwd_path = 1; fwd_kernel = "lstm_persistent";
         }
-        if (rc == 1) { rc = lstm_forward_stepwise(s, bufs, w, y, st); fwd_path = 0; }
+        if (rc == 1) { rc = lstm_forward_stepwise(s, bufs, w, y, st); fwd_path = 0; fwd_kernel = "lstm_step"; }
         B2_TRY(rc);
     }
     forward_done = true;
@@ -205,21 +205,21 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
             const bool single = lstm_single_supported(s, true);
             rc = single ? lstm_single_sweep(true, s, bufs, w, nullptr, dy, status_dev, st)
                         : lstm_cluster_sweep(true, s, bufs, w, nullptr, dy, status_dev, st);
-            bwd_path = single ? 1 : 7;
+            bwd_path = single ? 1 : 7; bwd_kernel = single ? "lstm_single" : "lstm_cluster";
         } else if (ptc_used && recurrence_mode != 6) {
             rc = lstm_ptc_sweep(true, s, bufs, ptc, w, nullptr, dy, status_dev, &tag_next, st);
-            bwd_path = 5;
+            bwd_path = 5; bwd_kernel = "lstm_ptc";
         } else if (wide_used) {
             rc = lstm_wide_sweep(true, s, bufs, wide, w, nullptr, dy, status_dev, &tag_next, st);
-            bwd_path = 5;
+            bwd_path = 5; bwd_kernel = "lstm_wide";
         }
         if (rc != 1) {
-        } else if (tcrec_used) { rc = lstm_backward_tc(s, bufs, tcrec, w, dy, status_dev, st); bwd_path = 3; }
+        } else if (tcrec_used) { rc = lstm_backward_tc(s, bufs, tcrec, w, dy, status_dev, st); bwd_path = 3; bwd_kernel = "lstm_step_tc"; }
         else if (recurrence_mode >= 1) {
             rc = lstm_persistent(true, persistent_transport(), s, bufs, w, nullptr, dy, xchg, status_dev, &tag_next, st);
-            bwd_path = 1;
+            bwd_path = 1; bwd_kernel = "lstm_persistent";
         }
-        if (rc == 1) { rc = lstm_backward_stepwise(s, bufs, w, dy, st); bwd_path = 0; }
+        if (rc == 1) { rc = lstm_backward_stepwise(s, bufs, w, dy, st); bwd_path = 0; bwd_kernel = "lstm_step"; }
         B2_TRY(rc);
     }
     const int NR = list ? n_list : N;      // frames the products run over
@@ -515,6 +515,11 @@ size_t b2_lstm_state_bytes(const b2_lstm *l) { return l ? l->impl.state_bytes : 
 int b2_lstm_recurrence_path(const b2_lstm *l, int backward) {
     if (!l) return -1;
     return backward ? l->impl.bwd_path : l->impl.fwd_path;
+}
+
+const char *b2_lstm_recurrence_kernel(const b2_lstm *l, int backward) {
+    if (!l) return "";
+    return backward ? l->impl.bwd_kernel : l->impl.fwd_kernel;
 }
 
 int b2_lstm_synchronize(b2_lstm *l, b2_stream st) {

@@ -45,9 +45,10 @@ struct LstmLayerImpl {
     bool want_cluster() const;
     bool want_ptc() const;
     int ensure_ptc();
-    // which recurrence the last forward / backward sweep actually ran: 0 one launch per timestep, 1 persistent
-    // FFMA kernels, 3 tensor-core GEMM + gate kernel per timestep, 5 persistent tensor-core kernels (512 units: lstm_ptc.cu, more: lstm_wide.cu), 7 register-resident cluster kernels
+    // which recurrence the last forward / backward sweep actually ran, as a family (b2_lstm_recurrence_path) and by the name of its source file
+    // (b2_lstm_recurrence_kernel): families 1 and 5 have two members each
     int fwd_path = -1, bwd_path = -1;
+    const char *fwd_kernel = "", *bwd_kernel = "";
     bool want_tc_recurrence() const;
     int ensure_tcrec();
     int check_status(cudaStream_t st);   // synchronises st; returns the kernels' status word

@@ -883,6 +883,12 @@ int b2_net_recurrence_path(b2_net *n, int layer, int backward) {
     if (!l) return -1;
     return backward ? l->impl().bwd_path : l->impl().fwd_path;
 }
+const char *b2_net_recurrence_kernel(b2_net *n, int layer, int backward) {
+    if (!n || layer < 0 || layer >= (int)n->net.layers.size()) return "";
+    LstmLayer *l = dynamic_cast<LstmLayer *>(n->net.layers[layer].get());
+    if (!l) return "";
+    return backward ? l->impl().bwd_kernel : l->impl().fwd_kernel;
+}
 int b2_net_set_recurrence_mode(b2_net *n, int mode) { if (!n) return B2_ERR_BAD_ARG; n->net.recurrenceMode = mode; return B2_OK; }
 int b2_net_set_force_ffma(b2_net *n, int on) { if (!n) return B2_ERR_BAD_ARG; n->net.forceFfma = on != 0; return B2_OK; }
 unsigned long long b2_net_launch_count(const b2_net *n) { return n ? g_launches - n->net.launchesAtCreate : 0; }

@@ -18,8 +18,8 @@ VARIANT_IDS = ["stepwise-ffma", "persistent-ffma", "persistent-tensor", "persist
                "stepwise-tensor", "persistent_l2-tensor"]
 
 
-def run_gpu(layers, P, lens, x, tg, weights, variant, lr=1e-4, mom=0.9, maxT=None, paths=None):
-    """paths: optional dict that receives {layer: (forward path, backward path)} of the (b)lstm layers"""
+def run_gpu(layers, P, lens, x, tg, weights, variant, lr=1e-4, mom=0.9, maxT=None, paths=None, kernels=None):
+    """paths, kernels: optional dicts that receive {layer: (forward, backward)} of the (b)lstm layers, path names resp. kernel files"""
     import b2lstm
     net = b2lstm.Net(layers, P, maxT or x.shape[0])
     net.set_recurrence_mode(variant["recurrence"])
@@ -43,6 +43,8 @@ def run_gpu(layers, P, lens, x, tg, weights, variant, lr=1e-4, mom=0.9, maxT=Non
     net.synchronize()
     if paths is not None:
         paths.update(net.recurrence_paths())
+    if kernels is not None:
+        kernels.update(net.recurrence_kernels())
     for i in weights:
         out["wnew%d" % i] = net.get_weights(i)
     out["launches"] = net.launch_count
@@ -195,8 +197,9 @@ def test_persistent_tensor_core_recurrence(ls, bi, P, lens, mode):
     x, tg = workloads.make_fraction(16, 8, P, lens, 51, 52)
     w = workloads.make_weights(layers, 53, 0.08)
     want = run_kind(checker(), layers, P, lens, x, tg, w)
-    paths = {}
-    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=mode, ffma=0), paths=paths)
+    paths, kernels = {}, {}
+    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=mode, ffma=0), paths=paths, kernels=kernels)
+    assert kernels[1] == ("lstm_ptc", "lstm_ptc" if mode == 5 else "lstm_persistent"), kernels
     assert paths[1][0] == "persistent_tensor_core", paths
     assert paths[1][1] == ("persistent_tensor_core" if mode == 5 else "persistent_ffma"), paths
     parity.compare_run(layers, got, want, "ls%d bi%d P%d" % (ls, bi, P), lstm_pad_zero_lens=lens)
@@ -361,7 +364,7 @@ def test_layer_level_entry_points_on_caller_buffers():
         pat[0, p] = 1
         pat[n - 1, p] = 3
     layer = b2lstm.LstmLayer(P, T, pls, ls, True, 1.0)
-    assert layer.num_weights == w[1].size
+    assert layer.num_weights == w[1].size and layer.recurrence_kernel() == ""
     tw, tx = torch.from_numpy(w[1]).to(dev), torch.from_numpy(x).to(dev)
     tpat = torch.from_numpy(pat).to(dev)
     ty = torch.full((T, P, ls), float("nan"), device=dev)
@@ -376,6 +379,7 @@ def test_layer_level_entry_points_on_caller_buffers():
     torch.cuda.synchronize()
     parity.assert_grads_close(layers, 1, tdw.cpu().numpy(), want["dw1"], "layer-level")
     assert np.isfinite(tdx.cpu().numpy()).all()
+    assert (layer.recurrence_kernel(), layer.recurrence_kernel(True)) == ("lstm_cluster", "lstm_cluster")
     layer.close()
 
 
@@ -547,8 +551,12 @@ def test_cluster_recurrence(els, bi, P, T):
     x, tg = workloads.make_fraction(7, 5, P, lens, 91, 92)
     w = workloads.make_weights(layers, 93, 0.2 if els < 100 else 0.08)
     want = run_kind(checker(), layers, P, lens, x, tg, w)
-    paths = {}
-    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0), paths=paths)
+    paths, kernels = {}, {}
+    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0), paths=paths, kernels=kernels)
+    # one or two (direction, sequence) pairs always find clusters of their own; from 19 on no device of 148 SMs has that many
+    pairs, some = P * (2 if bi else 1), ("lstm_cluster", "lstm_single")
+    for k, least in zip(kernels[1], (33, 129)):
+        assert k in (some[1:] if pairs <= 2 and els >= least else (some[:1] if pairs > 18 or els < least else some)), kernels
     if P > 16:   # fewer sequences: the FFMA kernels with one sequence per cluster may take a sweep
         assert paths[1] == ("cluster_tensor_core", "cluster_tensor_core"), paths
     parity.compare_run(layers, got, want, "els%d bi%d P%d" % (els, bi, P), lstm_pad_zero_lens=lens)
@@ -571,8 +579,9 @@ def test_wide_recurrence(els, bi, P, T):
     x, tg = workloads.make_fraction(7, 5, P, lens, 91, 92)
     w = workloads.make_weights(layers, 93, 0.08)
     want = run_kind(checker(), layers, P, lens, x, tg, w)
-    paths = {}
-    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0), paths=paths)
+    paths, kernels = {}, {}
+    got = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0), paths=paths, kernels=kernels)
+    assert kernels[1] == ("lstm_wide", "lstm_wide"), kernels
     assert paths[1] == ("persistent_tensor_core", "persistent_tensor_core"), paths
     parity.compare_run(layers, got, want, "els%d bi%d P%d" % (els, bi, P), lstm_pad_zero_lens=lens)
     again = run_gpu(layers, P, lens, x, tg, w, dict(recurrence=1, ffma=0))
