@@ -33,12 +33,10 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(ROOT, "project-currennt-public_b200"))
 
-# (workload, phase, recurrence path) -> DRAM bytes per cell-step (one unit, one frame slot) measured with ncu
+# (workload, phase, recurrence kernels) -> DRAM bytes per cell-step (one unit, one frame slot) measured with ncu
 TRAFFIC_BYTES_PER_CELL_STEP = {
-    ("cfg1", "lstm_fwd_recurrence", "persistent_ffma"): 26.1,
-    ("cfg1", "lstm_bwd_recurrence", "persistent_ffma"): 32.2,
-    ("cfg4", "lstm_fwd_recurrence", "persistent_tensor_core"): 38.2,
-    ("cfg4", "lstm_bwd_recurrence", "persistent_tensor_core"): 39.7,
+    ("cfg4", "lstm_fwd_recurrence", "lstm_wide"): 38.2,
+    ("cfg4", "lstm_bwd_recurrence", "lstm_wide"): 39.7,
 }
 
 METRIC = "blstm_train_step_frames_per_sec"
@@ -91,11 +89,12 @@ def workload_for(name, rank):
 
 
 # ---- algorithmic work per phase (per step, this rank) -----------------------------------------------
-def phase_work(layers, T, P, real_frames, count_padding=True):
+def phase_work(layers, lens):
     """{phase: (kind, amount)}: flops for GEMM phases, bytes for HBM phases (40 B forward / 44 B
-    backward per cell-step).  count_padding: over all T*P frame slots (what the kernels process) or
-    over the real frames only (the algorithmic work the roofline is quoted on)."""
-    N = T * P if count_padding else real_frames
+    backward per cell-step), over the real frames only, whatever a kernel does about padding: a phase
+    that leaves padding frames out is not credited with them, one that runs them has its useful work
+    counted.  The recurrent products pair every frame but a sequence's first."""
+    N, P = int(sum(lens)), len(lens)
     w = {}
 
     def add(k, kind, v):
@@ -118,7 +117,7 @@ def phase_work(layers, T, P, real_frames, count_padding=True):
             add("lstm_bwd_recurrence", "bytes", 44.0 * ls * N)
             add("lstm_fwd_recurrence_flops", "flops", 8.0 * ls * els * (N - P))
             add("lstm_bwd_recurrence_flops", "flops", 8.0 * ls * els * (N - P))
-            add("lstm_vector_grads", "bytes", 28.0 * ls * N)
+            add("lstm_vector_grads", "bytes", 20.0 * ls * N)    # four deltas, the cell state once
         elif ty == "sse":
             add("sse_loss", "bytes", 8.0 * ls * N)
             add("sse_grad", "bytes", 12.0 * ls * N)
@@ -431,7 +430,7 @@ def main():
         t = torch.tensor([real_frames], device="cuda", dtype=torch.float64)
         dist.all_reduce(t)
         frames_all = int(t.item())
-    rec_paths = net.recurrence_paths()
+    rec_paths, rec_kernels = net.recurrence_paths(), net.recurrence_kernels()
     check = None
     if world > 1 and not args.no_check:
         check = dp_correctness_record(net, wl, full if strong else None, rank, world, dist, torch, args)
@@ -440,12 +439,12 @@ def main():
 
     if rank == 0:
         pk = peaks()
-        work = phase_work(layers, T, P, real_frames)
+        work = phase_work(layers, lens)
         kernels = {}
         for name, (tms, ln) in prof.items():
             per = tms / args.steps
             ent = {"ms_per_step": round(per, 4), "launches_per_step": ln // args.steps, "share": round(tms / ms_prof, 4)}
-            if name in work and per > 0:
+            if name in work and ln:      # a phase may have nothing to launch (the deltas of an identity layer)
                 kind, amt = work[name]
                 if kind == "flops":
                     ent["tflops"] = round(amt / (per * 1e-3) / 1e12, 3)
@@ -456,7 +455,7 @@ def main():
                         ent["tflops"] = round(fl[1] / (per * 1e-3) / 1e12, 3)
             kernels[name] = ent
         top = max((k for k in kernels if k in work), key=lambda k: kernels[k]["ms_per_step"])
-        kind, amt = phase_work(layers, T, P, real_frames, count_padding=False)[top]   # real frames only
+        kind, amt = work[top]
         per_launch = kernels[top]["ms_per_step"] * 1e-3
         if kind == "flops":
             peak = pk["bf16"] / 3.0   # fp16 hi/lo split: three MMAs at the 16-bit rate per fp32 product
@@ -467,13 +466,13 @@ def main():
                     "peak_note": "%s copy bandwidth" % pk["src"]}
         roof["frac"] = roof["achieved"] / roof["peak"]
         # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per cell-step of the dominant kernel,
-        # per workload and recurrence path, from captures on reduced frame counts; traffic grows in proportion
+        # per workload and recurrence kernels, from captures on reduced frame counts; traffic grows in proportion
         # to the frame slots, so it is scaled by units x frame slots of one sweep of one layer.  None where no
         # capture of that kernel on that workload exists.
         path_fwd = sorted(set(v[0] for v in rec_paths.values()))
         path_bwd = sorted(set(v[1] for v in rec_paths.values()))
-        per_cell = TRAFFIC_BYTES_PER_CELL_STEP.get((args.workload, top, (path_fwd if "fwd" in top else path_bwd)[0]
-                                                    if (path_fwd and path_bwd) else ""))
+        kernels_ran = sorted(set(k["bwd" in top] for k in rec_kernels.values()))
+        per_cell = TRAFFIC_BYTES_PER_CELL_STEP.get((args.workload, top, "+".join(kernels_ran)))
         lstm_sizes = [l["size"] for l in layers if l["type"] in ("lstm", "blstm")]
         if per_cell and lstm_sizes and not args.ffma:
             roof["traffic"] = per_cell * (sum(lstm_sizes) / len(lstm_sizes)) * T * P
@@ -482,7 +481,8 @@ def main():
         else:
             roof["traffic"] = None
         roof["share_of_step"] = kernels[top]["share"]
-        in_b = int(x_host.numel() * 4 + t_host.numel() * 4 + T * P)
+        # inputs and targets; the lengths of up to 256 sequences travel as kernel arguments, of more as 2 P words
+        in_b = int(x_host.numel() * 4 + t_host.numel() * 4 + (8 * P if P > 256 else 0))
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
                 "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": scaling_of(args, world),
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -490,6 +490,7 @@ def main():
                            "real_frames_per_gpu_step": real_frames, "parallelism": "dp%d" % world,
                            "recurrence_mode_requested": args.recurrence,
                            "recurrence_forward": "+".join(path_fwd), "recurrence_backward": "+".join(path_bwd),
+                           "recurrence_kernels": sorted(set(k for v in rec_kernels.values() for k in v)),
                            "sequences_total": c["P"] if strong else P * world,
                            "gemm": "ffma" if args.ffma else "tcgen05_3xf16",
                            "frames_scale": args.frames_scale, "emulated_shard_of": args.shard_of,
