@@ -356,13 +356,12 @@ bool LstmLayerImpl::want_cluster() const {
     return !force_ffma && recurrence_mode == 1 && lstm_cluster_supported(shape()) && !want_wide();
 }
 
-// The persistent tensor-core kernels with weights in shared memory only serve 512 units per direction.  Modes 5 and 6 force them; the
-// default (mode 1) takes them where neither the kernels of lstm_wide.cu nor the cluster kernels fit the device.
+// The persistent tensor-core kernels with weights in shared memory only serve 512 units per direction, where modes 5 and 6 ask for them.
+// The default leaves them out: every device that holds their 64 co-resident blocks a direction holds a group of 16 of lstm_wide.cu, whose
+// step is shorter (512 units, 256 sequences 8.0 / 9.3 us against 11.1 / 13.5).  Their chains of 8 MMAs instead of 16 keep the
+// gradients a little closer to float64 (relative L2 4.8e-7 against 5.7e-7; outputs 5.3e-7 against 2.8e-7).
 bool LstmLayerImpl::want_ptc() const {
-    const LstmShape s = shape();
-    if (force_ffma || !lstm_ptc_supported(s)) return false;
-    if (recurrence_mode == 5 || recurrence_mode == 6) return true;
-    return recurrence_mode == 1 && s.P >= 16;
+    return !force_ffma && (recurrence_mode == 5 || recurrence_mode == 6) && lstm_ptc_supported(shape());
 }
 
 // The persistent tensor-core kernels with weights in shared and tensor memory, 257 to 1024 units per direction.
