@@ -1,6 +1,8 @@
 // What the recurrence kernels on thread-block clusters share (lstm_cluster.cu, lstm_single.cu, lstm_wide.cu): activations, bounded waits on
 // transaction barriers, sequence lengths.
 #pragma once
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -8,6 +10,15 @@ namespace b2 {
 namespace cluster {
 
 constexpr unsigned SPIN_LIMIT = 1u << 21;
+
+// fp32 values as two fp16 terms, x*S = hi + lo*2^-11; the scales of h (below 1) and of the gate deltas (clipped to [-1, 1])
+constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f, S_H = 16384.0f, S_D = 32768.0f;
+__device__ __forceinline__ uint32_t split_pair(float x, float S) {   // fp16 hi in the low half, lo in the high half
+    const float xs = x * S;
+    const __half h = __float2half_rn(xs);
+    const __half l = __float2half_rn((xs - __half2float(h)) * LO_SCALE);
+    return (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
+}
 
 // 1 / d, 1 <= d < 2^126: the hardware approximation (relative error e <= 2^-23) and one Newton step (r + r (1 - d r), relative error
 // e^2 before the last rounding): within 0.5001 ulp, without the division's branches
@@ -66,6 +77,44 @@ __device__ __forceinline__ float lds(uint32_t a) {
     return v;
 }
 __device__ __forceinline__ void sts(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+
+// A launch in clusters of `cluster` blocks (0: none), cooperative where blocks of different clusters wait for each other
+struct Launch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    Launch(int blocks, int threads, size_t smem, int cluster, bool cooperative, cudaStream_t st) {
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = attr;
+        if (cooperative) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
+            attr[cfg.numAttrs++].val.cooperative = 1;
+        }
+        if (cluster) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+            attr[cfg.numAttrs].val.clusterDim.x = cluster;
+            attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+            ++cfg.numAttrs;
+        }
+    }
+    Launch(const Launch &) = delete;
+    Launch &operator=(const Launch &) = delete;
+};
+// allows a kernel `smem` bytes of dynamic shared memory and, above 8, clusters of `cluster` blocks
+inline bool allow(const void *kern, size_t smem, int cluster) {
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                    (cluster <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess);
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+// clusters of a launch that the current device holds at once
+inline int resident(const void *kern, const Launch &l) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &l.cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    return n;
+}
 
 }  // namespace cluster
 }  // namespace b2

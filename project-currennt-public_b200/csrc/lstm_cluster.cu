@@ -47,8 +47,6 @@
 // other, so any number of them may be in flight or queued.
 #include <mutex>
 
-#include <cuda_fp16.h>
-
 #include "cluster.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
@@ -58,9 +56,6 @@ namespace {
 
 using namespace cluster;
 using namespace ptx;
-
-constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f;
-constexpr float S_H = 16384.0f, S_D = 32768.0f;
 
 constexpr int MAX_NT = 4;            // tiles a cluster runs in turn at most (kernels with weights in tensor memory)
 constexpr uint32_t TM_COLS = 256;    // tensor-memory columns for the lo parts: two warps a lane quarter, 128 columns each
@@ -78,12 +73,6 @@ struct ClusterArgs {
     int nclusters;
 };
 
-__device__ __forceinline__ uint32_t split_pair(float x, float S) {   // fp16 hi in the low half, lo in the high half
-    const float xs = x * S;
-    const __half h = __float2half_rn(xs);
-    const __half l = __float2half_rn((xs - __half2float(h)) * LO_SCALE);
-    return (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
-}
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t a0, const uint32_t a1, const uint32_t a2, const uint32_t a3,
                                          const uint32_t b0, const uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -671,18 +660,6 @@ const Variant BWD[] = {SHAPES(BWD_FULL) SHAPES_TM(BWD_TM)};
 constexpr int NFWD = (int)(sizeof(FWD) / sizeof(FWD[0])), NBWD = (int)(sizeof(BWD) / sizeof(BWD[0]));
 constexpr int NMAX = NFWD > NBWD ? NFWD : NBWD;
 
-void launch_config(const Variant &v, int nt, int clusters, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = v.C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    *cfg = cudaLaunchConfig_t{};
-    cfg->gridDim = dim3(clusters * v.C);
-    cfg->blockDim = dim3(32 * v.WN);
-    cfg->dynamicSmemBytes = v.smem(nt);
-    cfg->stream = st;
-    cfg->attrs = attr;
-    cfg->numAttrs = 1;
-}
-
 // clusters of a variant that the current device holds at once (asked once per kernel and device; *alone: with one block per SM, which
 // is also how many there are of the kernels that run several tiles)
 int resident_clusters(bool backward, int vi, int *alone) {
@@ -695,18 +672,9 @@ int resident_clusters(bool backward, int vi, int *alone) {
     short *k = known[dev][backward][vi];
     if (!k[0]) {
         const int spread = v.tm ? (int)v.smem(MAX_NT) : 120 * 1024;     // shared memory that keeps a second block off the SM
-        if (cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, spread) != cudaSuccess ||
-            (v.C > 8 && cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
-            cudaGetLastError();
-        for (int q = 0; q < 2; ++q) {
-            int n = 0;
-            cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute attr[1];
-            launch_config(v, 1, 1, nullptr, &cfg, attr);
-            if (q) cfg.dynamicSmemBytes = spread;
-            if (cudaOccupancyMaxActiveClusters(&n, v.kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-            k[q] = (short)(n + 1);
-        }
+        allow((const void *)v.kern, spread, v.C);
+        for (int q = 0; q < 2; ++q)
+            k[q] = (short)(1 + resident((const void *)v.kern, Launch(v.C, 32 * v.WN, q ? spread : v.smem(1), v.C, false, nullptr)));
     }
     *alone = k[1] - 1;
     return k[0] - 1;
@@ -801,10 +769,8 @@ int lstm_cluster_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, 
     ClusterArgs a;
     a.sh = s; a.bf = b; a.w = w; a.y = y; a.dy = dy; a.status = status;
     a.tiles = (s.P + 7) / 8; a.nt = pl.nt; a.n_items = pl.items; a.nclusters = pl.clusters;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    launch_config(v, pl.nt, pl.clusters, st, &cfg, attr);
-    B2_CUDA(cudaLaunchKernelEx(&cfg, v.kern, a));
+    const Launch l(pl.clusters * v.C, 32 * v.WN, v.smem(pl.nt), v.C, false, st);
+    B2_CUDA(cudaLaunchKernelEx(&l.cfg, v.kern, a));
     count_launch();
     return B2_OK;
 }

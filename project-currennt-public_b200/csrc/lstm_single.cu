@@ -434,17 +434,6 @@ constexpr Variant variant() {
 const Variant VARIANTS[] = {variant<8, 16, false>(), variant<16, 16, false>(), variant<16, 32, true>()};
 constexpr int NVARIANTS = (int)(sizeof(VARIANTS) / sizeof(VARIANTS[0]));
 
-void launch_config(const Variant &v, bool backward, int clusters, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = v.C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    *cfg = cudaLaunchConfig_t{};
-    cfg->gridDim = dim3(clusters * v.C);
-    cfg->blockDim = dim3(NTHR);
-    cfg->dynamicSmemBytes = backward ? v.smem_b : v.smem_f;
-    cfg->stream = st;
-    cfg->attrs = attr;
-    cfg->numAttrs = 1;
-}
 // clusters of a variant that the current device holds at once with one block per SM (asked once per kernel and device)
 int resident_clusters(bool backward, int vi) {
     static std::mutex mu;
@@ -456,18 +445,8 @@ int resident_clusters(bool backward, int vi) {
     if (!k) {
         const Variant &v = VARIANTS[vi];
         const Kernel f = backward ? v.bwd : v.fwd;
-        int n = 0;
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[1];
-        launch_config(v, backward, 1, nullptr, &cfg, attr);
-        cfg.dynamicSmemBytes = 120 * 1024;     // keeps a second block off the SM
-        if (cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024) != cudaSuccess ||
-            (v.C > 8 && cudaFuncSetAttribute((const void *)f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-            cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
-        k = (short)(n + 1);
+        const size_t spread = 120 * 1024;      // keeps a second block off the SM
+        k = (short)(1 + (allow((const void *)f, spread, v.C) ? resident((const void *)f, Launch(v.C, NTHR, spread, v.C, false, nullptr)) : 0));
     }
     return k - 1;
 }
@@ -494,10 +473,8 @@ int lstm_single_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, c
     SingleArgs a;
     a.sh = s; a.bf = b; a.w = w; a.y = y; a.dy = dy; a.status = status;
     a.n_items = a.nclusters = s.D * s.P;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    launch_config(v, backward, a.nclusters, st, &cfg, attr);
-    B2_CUDA(cudaLaunchKernelEx(&cfg, backward ? v.bwd : v.fwd, a));
+    const Launch l(a.nclusters * v.C, NTHR, backward ? v.smem_b : v.smem_f, v.C, false, st);
+    B2_CUDA(cudaLaunchKernelEx(&l.cfg, backward ? v.bwd : v.fwd, a));
     count_launch();
     return B2_OK;
 }

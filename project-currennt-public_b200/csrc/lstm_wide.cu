@@ -38,8 +38,6 @@
 // most 16 main products (tensor-memory accumulation truncates).
 //
 // Blocks of a group wait for each other, so the launch is cooperative.  Every wait is bounded as in lstm_ptc.cu.
-#include <cuda_fp16.h>
-
 #include <algorithm>
 #include <mutex>
 
@@ -54,6 +52,10 @@ using namespace ptx;
 using cluster::cl_logistic;
 using cluster::cl_tanh;
 using cluster::settle;
+using cluster::split_pair;
+using cluster::LO_UNSCALE;
+using cluster::S_D;
+using cluster::S_H;
 
 constexpr int KB = 8;                                     // operand images of a slice
 // Step counters: a line of 128 bytes for each slice (fewer readers wait longer for a line that many SMs poll: one line for all slices,
@@ -62,7 +64,6 @@ constexpr int KB = 8;                                     // operand images of a
 constexpr int LINE = 32, GROUP_FLAGS = (16 + 8) * LINE;
 constexpr long long WAIT_CYCLES = 4000000000LL;
 constexpr unsigned POLL_LIMIT = 1u << 22;
-constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f, S_H = 16384.0f, S_D = 32768.0f;
 constexpr int W_POLL = 0, W_MMA = 1;
 constexpr uint32_t A_BYTES = 131072;
 
@@ -106,12 +107,6 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, u64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
         "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-__device__ __forceinline__ uint32_t split_pair(float x, float S) {   // fp16 hi in the low half, lo in the high half
-    const float xs = x * S;
-    const __half h = __float2half_rn(xs);
-    const __half l = __float2half_rn((xs - __half2float(h)) * LO_SCALE);
-    return (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
 }
 
 // the end of a round of polling; every lane of the warp leaves in the same round
@@ -619,19 +614,6 @@ constexpr Variant variant_of() {
 #define CHUNKS(E, BWD) {variant_of<E, BWD, 16>(), variant_of<E, BWD, 32>(), variant_of<E, BWD, 64>()}
 const Variant VARIANTS[2][2][NVARIANTS] = {{CHUNKS(512, false), CHUNKS(512, true)}, {CHUNKS(1024, false), CHUNKS(1024, true)}};   // [wide][backward]
 
-void launch_config(const Variant &v, int groups, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute (*attr)[2]) {
-    (*attr)[0].id = cudaLaunchAttributeCooperative;
-    (*attr)[0].val.cooperative = 1;
-    (*attr)[1].id = cudaLaunchAttributeClusterDimension;
-    (*attr)[1].val.clusterDim.x = v.cluster; (*attr)[1].val.clusterDim.y = 1; (*attr)[1].val.clusterDim.z = 1;
-    *cfg = cudaLaunchConfig_t{};
-    cfg->gridDim = dim3(groups * v.group);
-    cfg->blockDim = dim3(v.threads);
-    cfg->dynamicSmemBytes = v.smem;
-    cfg->stream = st;
-    cfg->attrs = *attr;
-    cfg->numAttrs = v.cluster > 1 ? 2 : 1;
-}
 // groups that the current device holds at once, at most those the exchange buffers are made for
 constexpr int MAX_GROUPS[2] = {8, 2};
 int resident_groups(bool wide) {
@@ -644,15 +626,8 @@ int resident_groups(bool wide) {
         int groups = std::min(MAX_GROUPS[wide], sm_count() / VARIANTS[wide][0][0].group);
         for (int i = 0; wide && i < NVARIANTS; ++i) {
             const Variant &v = VARIANTS[wide][0][i];
-            int n = 0;
-            cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute attr[2];
-            launch_config(v, 1, nullptr, &cfg, &attr);
-            if (cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem) != cudaSuccess ||
-                cudaOccupancyMaxActiveClusters(&n, v.kern, &cfg) != cudaSuccess) {
-                cudaGetLastError();
-                n = 0;
-            }
+            const cluster::Launch l(v.group, v.threads, v.smem, v.cluster, true, nullptr);
+            const int n = cluster::allow((const void *)v.kern, v.smem, v.cluster) ? cluster::resident((const void *)v.kern, l) : 0;
             groups = std::min(groups, v.cluster * n / v.group);
         }
         known[dev][wide] = (short)(groups + 1);
@@ -702,10 +677,8 @@ int lstm_wide_sweep(bool backward, const LstmShape &s, const LstmBuffers &b, con
     a.tag_base = *tag_next;
     a.nchunks = pl.nchunks;
     B2_TRY(set_max_dynamic_smem((const void *)v.kern, (int)v.smem));
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[2];
-    launch_config(v, pl.groups, st, &cfg, &attr);
-    B2_CUDA(cudaLaunchKernelEx(&cfg, v.kern, a));
+    const cluster::Launch l(pl.groups * v.group, v.threads, v.smem, v.cluster > 1 ? v.cluster : 0, true, st);
+    B2_CUDA(cudaLaunchKernelEx(&l.cfg, v.kern, a));
     count_launch();
     *tag_next += (unsigned)(s.D * a.nchunks) * ((unsigned)s.T + 1u);
     return B2_OK;
