@@ -35,6 +35,8 @@ sys.path.insert(0, os.path.join(ROOT, "project-currennt-public_b200"))
 
 # (workload, phase, recurrence kernels) -> DRAM bytes per cell-step (one unit, one frame slot) measured with ncu
 TRAFFIC_BYTES_PER_CELL_STEP = {
+    ("cfg1", "lstm_fwd_recurrence", "lstm_cluster"): 26.0,
+    ("cfg1", "lstm_bwd_recurrence", "lstm_cluster"): 29.3,
     ("cfg4", "lstm_fwd_recurrence", "lstm_wide"): 38.2,
     ("cfg4", "lstm_bwd_recurrence", "lstm_wide"): 39.7,
 }

@@ -116,20 +116,19 @@ int b2_lstm_backward(b2_lstm *layer, const float *weights_dev, const float *x_de
                      const float *dy_dev, float *dx_dev, float *dw_dev, b2_stream stream);
 /* Which recurrence kernels run:
  *   0  one launch per timestep;
- *   1  persistent kernels, the library chooses the exchange between the blocks of a group (default):
- *      thread-block clusters with transaction barriers in distributed shared memory for as many work
- *      items as fit side by side, the remaining sequences through L2 on the SMs the clusters leave
- *      free; up to 320 units per direction tensor-core kernels with the weights in registers; for large batches (many
- *      sequences x many units) the tensor-core recurrence of mode 3;
- *   2  persistent kernels, every group as a cluster where a group fits one (128 or 256 units per
- *      direction), through L2 otherwise;
- *   3  tensor-core recurrence (one batched tcgen05 GEMM and one gate kernel per timestep) wherever
- *      the shape allows it;
- *   4  persistent kernels, every exchange through L2;
- *   5  persistent tensor-core kernels (recurrent weights resident in shared memory as fp16 hi/lo tcgen05 operands for
- *      the whole sweep) wherever the shape allows it (512 units per direction); mode 1 picks them by itself from 16
- *      parallel sequences on;
- *   6  as 5 for the forward sweep only (the backward sweep runs on the mode-1 kernels). */
+ *   1  the library's choice (default), one launch per sweep up to 1024 units per direction:
+ *      - up to 512 units, thread-block clusters with the recurrent weights in registers (and tensor memory): fp32 FFMA with one
+ *        sequence per cluster where every (direction, sequence) finds a cluster of its own, tensor-core products otherwise;
+ *      - 257 to 512 units with many sequences and 513 to 1024 units, tensor-core kernels with the weights in shared and tensor memory;
+ *      - 1024 units with one sequence (one direction: up to 8), the FFMA kernels of modes 2 and 4;
+ *      - above 1024 units the kernels of mode 3 from 16 sequences on, otherwise one launch per timestep;
+ *   2  persistent FFMA kernels of 128, 256, 512 or 1024 units per direction, every group of blocks as a thread-block cluster where a
+ *      group fits one (128 or 256 units), through L2 otherwise; other unit counts one launch per timestep;
+ *   3  tensor-core recurrence (one batched tcgen05 GEMM and one gate kernel per timestep) wherever the shape allows it;
+ *   4  as 2, every exchange through L2;
+ *   5  persistent tensor-core kernels with the weights in shared memory only (512 units per direction; mode 1 never picks them);
+ *   6  as 5 for the forward sweep only (the backward sweep runs on the persistent FFMA kernels).
+ * With strict fp32 products (b2_net_set_force_ffma) every mode but 0 runs the FFMA kernels of modes 2 and 4. */
 int b2_lstm_set_recurrence_mode(b2_lstm *layer, int mode);
 /* Which recurrence kernels the layer's last forward (backward = 0) or backward (backward != 0) sweep really
  * ran, whatever the mode asked for: 0 one launch per timestep, 1 persistent FFMA kernels, 3 tensor-core GEMM
@@ -158,7 +157,7 @@ typedef struct b2_net b2_net;
  * "learningRate"?}, ...], "weights"?: {name: {"input":[..],"bias":[..],"internal":[..]}}}),
  * NeuralNetwork.cpp:1056-1086, TrainableLayer.cu:135-205.  Layer types understood: input,
  * feedforward_tanh, feedforward_logistic, feedforward_identity, lstm, blstm, sse.
- * Weights absent from the JSON are drawn U(-0.08, 0.08)... by seed `random_seed`. */
+ * Weights absent from the JSON are drawn by seed `random_seed` (range: b2_config_set_weights_uniform). */
 int b2_net_create(const char *network_json, int parallel_sequences, int max_seq_length, unsigned random_seed,
                   b2_net **out);
 /* --lstm_forget_gate_bias (Configuration.cpp:682-683, layers/LstmLayer.cu:1147-1161): a value above 1e-4 is added to
@@ -172,7 +171,7 @@ void b2_config_set_lstm_forget_gate_bias(float value);
  * Process-wide; call before b2_net_create. */
 void b2_config_set_weights_uniform(float min, float max);
 
-/* Tuning of the persistent tensor-core recurrence (no counterpart in the reference).  The sequences of a fraction are
+/* Tuning of the persistent tensor-core recurrence of modes 5 and 6 (no counterpart in the reference).  The sequences of a fraction are
  * processed in chunks of 32 or 64; the chunks of a group of blocks are in flight together.
  *   nc32_chunks: the largest number of chunks per group for which chunks are 32 sequences wide and use the
  *     latency-optimised exchange (self-validating words through L2 instead of step counters and bulk copies);
@@ -266,8 +265,8 @@ int b2_net_synchronize(b2_net *net);
 /* The stream all of the net's work is ordered on (a cudaStream_t). */
 b2_stream b2_net_stream(b2_net *net);
 /* The recurrence mode of every (b)lstm layer, values as for b2_lstm_set_recurrence_mode: 0 stepwise,
- * 1 persistent kernels of the library's choice (default), 2 clusters, 3 tensor-core GEMM per step,
- * 4 L2 only, 5 persistent tensor-core kernels, 6 those for the forward sweep only. */
+ * 1 the library's choice (default), 2 FFMA kernels on clusters, 3 tensor-core GEMM per step, 4 FFMA kernels
+ * through L2, 5 tensor-core kernels with weights in shared memory, 6 those for the forward sweep only. */
 int b2_net_set_recurrence_mode(b2_net *net, int mode);
 /* b2_lstm_recurrence_path of layer `layer` of the net; -1 for layers that are no (b)lstm. */
 int b2_net_recurrence_path(b2_net *net, int layer, int backward);

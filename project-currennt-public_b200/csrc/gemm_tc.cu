@@ -23,9 +23,10 @@
 // one cross term side by side), a_lo x b_hi another (N=128, onto the cross columns), and releases slots with tcgen05.commit;
 // warps 2-9 (two per tensor-memory lane quarter, half of the tile's columns each) drain the double-buffered accumulator pair from TMEM
 // with tcgen05.ld every SEG slabs, add the segments in registers and finally write C.
-// What bounds it: shared memory.  A slab costs the tensor core 768 cycles; three N=128 products read 96 KB of operands for it and TMA
-// writes 64 KB, 1280 cycles at 128 bytes per cycle; with the wide instruction the products read 80 KB (1152).
-// B200, 8192 x 64000 x 2048: 6.5 -> 5.9 ms, 1.09 PFLOP/s counting all three products.  Operands may be K-major (k
+// What bounds it: shared memory.  A slab costs the tensor core 768 cycles; with the wide instruction its products read 80 KB of
+// operands (640 wavefronts of 128 bytes, three N=128 products 96 KB) while TMA writes 64 KB.  Measured 1073 to 1112 cycles a slab on long
+// contractions (tensor pipe 72 to 69 % active), 1387 at K = 512, where draining a tile is not hidden.
+// B200, 8192 x 64000 x 2048 with the split of its operands: 6.5 -> 5.8 ms, 1.1 PFLOP/s counting all three products.  Operands may be K-major (k
 // contiguous) or MN-major (m resp. n contiguous); MN-major tiles are fetched as column blocks one
 // swizzle row wide so that they land in the canonical MN-major SWIZZLE_128B layout.  Optional split-K over
 // gridDim.z into scratch (summed by a second kernel in a fixed order).

@@ -12,8 +12,9 @@
 // whatever N is (lstm_ptc.cu); here the weights sit in the registers of the warps that own them, and a warp-level MMA of 16 x 16
 // weights with 8 sequences takes 8 cycles of its tensor core: 256 units, 8 sequences on 8 SMs are 768 cycles, against 2048 of FFMA.
 // Measured (B200, us per step forward / backward, against the FFMA kernels of lstm_persistent.cu or, for unit counts those do not
-// have, one launch per step): 256 units per direction, 32 sequences 1.27 / 1.27 (1.74 / 1.56), 4 sequences 0.78 / 1.01 (1.74 / 1.40),
-// 128 sequences 3.6 / 3.8 (6.0 / 5.8); 128 units, 1 sequence 0.66 / 0.81 (1.28 / 0.99); 160 units, 8 sequences 0.95 / 1.0 (20 / 57).
+// have, one launch per step): 256 units per direction, 32 sequences 1.17 / 1.18 (1.74 / 1.56), 4 sequences 0.75 / 0.91 (1.74 / 1.40),
+// 128 sequences 3.6 / 3.6 (6.0 / 5.8); 128 units, 16 sequences 0.68 / 0.74; 160 units, 8 sequences 0.94 / 0.94 (20 / 57); a sweep
+// takes 5 to 30 us besides (launch, weights).  ncu, 256 units, 32 sequences: tensor pipe 32 % of the cycles, DRAM 0.36 TB/s.
 //
 // Decomposition.  Block b of a cluster of C owns U = 4*WN hidden units with all four gates; its WN warps own 4 units (16 gate
 // rows, one m-tile) each.  Unit counts that do not fill C*U are padded with zero weights; the padding units' outputs are 0.
@@ -28,8 +29,8 @@
 //
 // Above 320 units (TM): a block's 65536 weights are twice the register file.  The fp16 hi parts stay in registers, the lo parts in tensor
 // memory, from where a warp reads the fragments of four k-steps while it multiplies those before.  Here the product (1536 cycles of
-// the tensor cores a tile) is long enough for a second tile to hide the exchange: 512 units, 32 sequences 3.3 / 4.0 us (4.1 / 4.9 with
-// lstm_ptc.cu), one direction of 50 sequences 2.1 / 2.1 (4.1 / 4.9), 384 units and 8 sequences 1.5 / 1.65 (38 / 125, a launch per step).
+// the tensor cores a tile) is long enough for a second tile to hide the exchange: 512 units, 32 sequences 3.2 / 3.9 us (4.1 / 4.9 with
+// lstm_ptc.cu), one direction of 50 sequences 2.0 / 2.0 (4.1 / 4.9), 384 units and 8 sequences 1.4 / 1.6 (38 / 125, a launch per step).
 //
 // Tried and dropped: several tiles per cluster in turn where all weights are in registers (the second tile costs as much as the first:
 // a warp's own instruction stream, not the exchange, is what fills its time); inputs through a cp.async ring (0.13 us per step more than plain loads).
@@ -756,7 +757,7 @@ bool lstm_cluster_supported(const LstmShape &s) { return s.els <= 512 && make_pl
 
 // The fit of step_cycles holds up to 256 units; beyond, several tiles in turn and 16 blocks a cluster, measured steps are 1.4 times as long
 // (us per step, forward + backward, estimated and measured: 512 units, 64 sequences, bidirectional 7.8 and 11.5, 32 sequences 5.9 and
-// 7.9; 400 units, 128 sequences 15.7 and 23.8; 300 units, 64 sequences 6.5 and 8.8).
+// 7.1; 400 units, 128 sequences 15.7 and 23.8; 300 units, 64 sequences 6.5 and 8.8).
 double lstm_cluster_step_us(const LstmShape &s) {
     return (s.els > 256 ? 1.4 : 1.0) * (make_plan(s, false).cycles + make_plan(s, true).cycles) / 1950.0;
 }

@@ -329,10 +329,10 @@ int LstmLayerImpl::backward(const float *w, const float *x, const float *y, cons
     return B2_OK;
 }
 
-// Which recurrence runs.  Mode 3 forces the tensor-core recurrence where the shape allows it; the
-// default (mode 1) picks it when the persistent kernel would need many passes of expensive steps:
-// measured on B200 a persistent step costs about 1.4 us + 0.27 us per sequence of a work item, a
-// tensor-core step (GEMM + gate kernel, two launches) about 10 us whatever the batch.
+// Which recurrence runs.  Mode 3 forces the tensor-core recurrence where the shape allows it; the default (mode 1) asks here only
+// where neither the cluster kernels nor those of lstm_wide.cu serve the shape (above 1024 units, or a device that holds neither), and
+// picks it when the persistent kernel would need many passes of expensive steps: measured on B200 a persistent step costs about 1.4 us
+// + 0.27 us per sequence of a work item, a tensor-core step (GEMM + gate kernel, two launches) about 10 us whatever the batch.
 bool LstmLayerImpl::want_tc_recurrence() const {
     const LstmShape s = shape();
     if (force_ffma || !lstm_tc_supported(s) || (desc.size % 4) != 0) return false;
@@ -366,7 +366,7 @@ bool LstmLayerImpl::want_ptc() const {
 
 // The persistent tensor-core kernels with weights in shared and tensor memory, 257 to 1024 units per direction.
 // Up to 512 units they take the fractions whose sequences need several passes of the cluster kernels (B200, us per step forward / backward,
-// bidirectional, cluster kernels and these: 512 units, 32 sequences 3.8 / 4.0 and 4.5 / 5.9, 64: 5.5 / 5.9 and 4.5 / 6.0, 128: 9.3 / 10.1 and
+// bidirectional, cluster kernels and these: 512 units, 32 sequences 3.2 / 3.9 and 4.5 / 5.9, 64: 5.5 / 5.9 and 4.5 / 6.0, 128: 9.3 / 10.1 and
 // 5.7 / 6.9, 256: 16.2 / 19.8 and 8.0 / 9.3; 300 units, 64: 4.0 / 4.8 and 4.4 / 5.9, 128: 7.6 / 9.5 and 5.8 / 6.9).
 // Few sequences of 1024 units are left to the FFMA kernels (lstm_persistent.cu), whose step is shorter while one pass of 8 sequences (or
 // one sequence per direction) covers the fraction (one sequence, bidirectional 3.6 / 3.4 there, 4.6 / 5.9 here; unidirectional 1 to 8

@@ -9,7 +9,7 @@ struct LstmLayerImpl {
     int D = 1, els = 0;
     int T = 0, Tmin = 0;
     bool forward_done = false;
-    int recurrence_mode = 1;   // 0 stepwise, 1 persistent
+    int recurrence_mode = 1;   // b2_lstm_set_recurrence_mode
     bool force_ffma = false;
     float x_bound = 0.0f;         // > 0: no |entry| of the layer's input exceeds it (the layer stack knows its layers' ranges)
     bool check_padding = false;   // load_sequences verifies that padding frames trail their sequences
@@ -29,8 +29,7 @@ struct LstmLayerImpl {
     unsigned tag_next = 1;
     // tensor-core recurrence (large batches): hi/lo buffers, allocated on first use
     TcRecBuffers tcrec{};
-    // recurrence mode 1 lets the library choose, 2 forces clusters, 4 forces L2, 5 the persistent tensor-core
-    // kernels, 6 those for the forward sweep only
+    // of lstm_persistent.cu: mode 2 forces clusters, 4 forces L2
     int persistent_transport() const { return recurrence_mode == 2 ? 1 : (recurrence_mode == 4 ? 0 : 2); }
     bool tcrec_used = false;      // this fraction's forward sweep ran on the tensor-core recurrence
     // persistent tensor-core recurrence: weight images, exchange words (allocated on first use)

@@ -1,5 +1,6 @@
 // Persistent LSTM recurrence kernels: ONE launch runs all timesteps of a layer's forward (or
-// BPTT backward) sweep, both directions concurrently.
+// BPTT backward) sweep, both directions concurrently.  The default takes them for 1024 units per direction with few sequences and for
+// strict fp32 products; elsewhere lstm_cluster.cu, lstm_single.cu and lstm_wide.cu replaced them.
 //
 // Replaces the reference's per-timestep loop of 4 cublasSgemm + 1 Thrust functor per direction
 // (layers/LstmLayer.cu:1805-1858,1878-1927 forward with ComputeBlockOutputFn :57-185;
@@ -25,9 +26,9 @@
 // sums of the k-ranges (row ranges) are combined through shared memory.
 //
 // Exchange.  Two transports, same data flow:
-//  * thread-block cluster (groups of <= 8 blocks: 128 or 256 units per direction): values are stored
-//    straight into the peers' shared memory (distributed shared memory, st.shared::cluster) and one
-//    hardware cluster barrier (arrive.release / wait.acquire) per step orders them;
+//  * thread-block cluster (groups of <= 8 blocks: 128 or 256 units per direction): values go straight into the peers'
+//    shared memory with st.async, which counts their bytes on a transaction barrier the receiver polls; a hardware
+//    cluster barrier only between work items;
 //  * L2 (any group size): the flag travels inside the datum: one naturally aligned 64-bit word
 //    {step tag : float bits}, written with st.relaxed.gpu and polled with ld.relaxed.gpu, so one L2
 //    round trip delivers both "ready" and the value; no fence, no atomics.  Polling goes in rounds

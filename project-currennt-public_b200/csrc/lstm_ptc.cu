@@ -1,6 +1,7 @@
 // Persistent tensor-core recurrence: ONE launch runs all timesteps of a (b)lstm layer's forward sweep (a second
 // one the BPTT sweep) for any number of parallel sequences, with the recurrent weights RESIDENT in shared memory
-// as tcgen05 operands for the whole sweep.
+// as tcgen05 operands for the whole sweep.  Recurrence modes 5 and 6 run them (512 units per direction); the default takes lstm_cluster.cu
+// and lstm_wide.cu, whose steps are shorter.
 //
 // Replaces the reference's loop of 4 cublasSgemm + 1 Thrust functor per timestep and direction
 // (layers/LstmLayer.cu:1805-1858,1878-1927 forward with ComputeBlockOutputFn :57-185; :2115-2176,2195-2253

@@ -10,7 +10,7 @@
 // one per 16 bytes received), reductions and cell math.  65536 fp32 weights fill the register file, so half of them live in TENSOR
 // MEMORY, which nothing else uses here: each thread reads its 128 words back with tcgen05.ld while the register half is multiplied
 // (512 bytes per cycle and SM: half the time of the FFMAs).  Through L2 with 32 blocks per direction (lstm_persistent.cu) a step of
-// 512 units took 1.60 / 1.43 us forward / backward, here 1.03 / 1.02 (256 units: 1.36 / 1.03 there, 0.75 / 0.87 here).
+// 512 units took 1.60 / 1.43 us forward / backward, here 1.01 / 0.95 (256 units: 1.36 / 1.03 there, 0.84 / 0.80 here).
 //
 //   forward : warp w of 8 owns U/8 units x 4 gates (rows) of the block; a lane takes KP/32 source units of every row, a transposing
 //             butterfly of shuffles leaves one row sum per lane group; the gates' activations run in different lanes, shuffles bring
@@ -460,7 +460,9 @@ int pick_variant(int els) {
 
 // Every (direction, sequence) needs a cluster of its own with one block per SM (7 clusters of 16, 15 of 8 on a B200); blocks that
 // share an SM lose to the 8-column tiles of lstm_cluster.cu (128 units, 16 pairs: 0.73 us per step against 0.69).  Forward from 33
-// units on (below, one block without an exchange is faster), backward from 129 on (128 units: 0.79 us against 0.73 of lstm_cluster.cu).
+// units on (below, one block without an exchange is faster; 128 units 0.57 us a step, 512 units 1.01 against 1.33 of lstm_cluster.cu; at 256
+// units this side of the line is the slower one, 0.84 against 0.75), backward from 129 on (128 units: 0.79 us against 0.72 of
+// lstm_cluster.cu; 256 units 0.80 against 0.91, 512 units 0.95 against 1.91).
 bool lstm_single_supported(const LstmShape &s, bool backward) {
     const int vi = pick_variant(s.els);
     return vi >= 0 && s.els > (backward ? 128 : 32) && s.D * s.P <= resident_clusters(backward, vi);

@@ -2,9 +2,8 @@
 // both directions) for the recurrent product and ONE fused gate kernel.
 //
 // Same arithmetic as the reference's time loops (layers/LstmLayer.cu:1805-1858,1878-1927 forward,
-// :2115-2176,2195-2253 backward: 4 cublasSgemm + one Thrust functor per step and direction), used
-// when parallel_sequences x units is large enough that the per-step product (4*els x els x P) belongs
-// on the tensor cores; the persistent FFMA kernels (lstm_persistent.cu) win when it is small.
+// :2115-2176,2195-2253 backward: 4 cublasSgemm + one Thrust functor per step and direction), used from 16
+// sequences on above 1024 units per direction, whose weights no persistent kernel here holds, and in recurrence mode 3.
 //
 //   forward  step: rec[d][p][g*els+j]  = sum_k W_rec[g][d][j][k] * h_d[prev][p][k]     (3xTF32 GEMM,
 //                  batches = (direction, gate), K split over blocks, partial sums to scratch)

@@ -31,8 +31,8 @@
 // per step forward / backward: one thread issuing all MMAs and a proxy fence before each bulk copy 12.7 / 16.8; several issuers (a
 // tcgen05.mma with run-time descriptors costs its thread 118 cycles) and one fence on the publishing side 10.3 / 14.0; copies issued by 8
 // lanes side by side and the layer's state stored only after the publication 8.4 / 11.8; the counters on lines of their own and
-// partial sums read straight from L2 7.6 / 7.7.  512 units, 256 sequences in eight groups: 8.0 / 9.3, of which the cells of 32 units x 64
-// sequences take 2 (lstm_ptc.cu 11.1 / 13.5).  The launch pair per step of lstm_step_tc.cu takes 24.6 / 26.6; 16 sequences: 4.5 / 6.0
+// partial sums read straight from L2 7.6 / 7.8 (at 1.95 GHz; four layers under the power cap at 1.6 GHz 8.9 / 10.2).  512 units, 256 sequences in eight groups: 8.2 / 9.4, of which the cells of 32 units x 64
+// sequences take 2 (lstm_ptc.cu 11.1 / 13.5).  The launch pair per step of lstm_step_tc.cu takes 24.6 / 26.6; 16 sequences: 4.3 / 5.7
 // and 23.0 / 23.8.
 // Numerics as in lstm_ptc.cu: x*S = hi + lo*2^-11, S = 2^14 for h, 2^15 for the deltas, 2^13 <= max|w|*S < 2^14 per block; a chain holds at
 // most 16 main products (tensor-memory accumulation truncates).
